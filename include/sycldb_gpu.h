@@ -245,8 +245,11 @@ int sdb_compact_gather_occ(const uint32_t *occ, uint64_t n, int ncols, const voi
  * ... (nkeys <= 16; key_types[k] 0 = int32 compared signed, 1 = uint64
  * compared unsigned, the comparisons of the reference's sort_table,
  * kernels/sort.hpp:7-103; descending[k] != 0 reverses key k).  Stable: equal
- * rows keep their order.  n <= 2^31.  A radix sort: 4 passes per int32 key,
- * 8 per uint64 key.  scratch: sdb_sort_scratch_bytes(n) bytes, 256-byte aligned.
+ * rows keep their order.  n <= 2^31.  Small inputs by counting, others by a
+ * radix sort of the keys' first 32 varying bits, or of all their digits where
+ * those do not decide the order.  scratch: sdb_sort_scratch_bytes(n) bytes,
+ * 256-byte aligned.  Should a bounded wait inside the sort run out, perm is
+ * 0..n-1 and sdb_device_errors counts it.
  * The reference's executor itself treats SORT as a pass-through
  * (executor/ddor_executor.cpp:209-211). */
 size_t sdb_sort_scratch_bytes(uint64_t n);

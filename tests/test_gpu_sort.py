@@ -60,3 +60,25 @@ def test_sort_argument_checks():
     assert L.sdb_sort_rows(ptrs, types, dsc, 1, 10, 0x2000, 0x3000, 16, None) == capi.SDB_ERR_INVALID  # scratch
     assert L.sdb_sort_rows(ptrs, types, dsc, 0, 10, 0x2000, 0x3000, 1 << 20, None) == capi.SDB_ERR_INVALID
     assert L.sdb_sort_rows(ptrs, types, dsc, 1, 0, 0x2000, 0x3000, 1 << 20, None) == capi.SDB_OK  # nothing to do
+
+
+@pytest.mark.parametrize("n", [4096, 4097, 6144, 6145, 12_289, 262_144, 262_145, 5_000_000])
+def test_sort_across_the_small_input_and_tile_edges(n):
+    """The counting path's last sizes, the radix path's first, partial last
+    tiles, more tiles than run at once; keys whose high bytes are the same in
+    every row (dropped passes), an even and an odd number of passes left."""
+    rng = np.random.default_rng(n)
+    year = rng.integers(1992, 1999, n).astype(np.int32)
+    total = rng.integers(0, 2**40, n).astype(np.uint64)
+    wide = rng.integers(-2**31, 2**31 - 1, n, dtype=np.int64).astype(np.int32)
+    same = np.full(n, 7, np.int32)
+    # few heads although each digit of a head is evenly spread: tied runs too long to order one by one
+    b = rng.integers(0, 256, n).astype(np.uint64)
+    deep = sum((b << np.uint64(8 * q) for q in range(2, 8)), rng.integers(0, 2**16, n).astype(np.uint64))
+    skew = np.where(rng.random(n) < 0.9, 5, wide).astype(np.int32)  # one value in most rows
+    for keys, desc in (([year, total], [False, True]), ([wide], [True]), ([same, year], [True, False]),
+                       ([year], [False]), ([same, same], [False, True]), ([year, deep], [False, True]),
+                       ([skew, wide], [True, False])):
+        got = gpu_sort(keys, desc)
+        want = np.lexsort([sortable(k, d) for k, d in reversed(list(zip(keys, desc)))])
+        assert np.array_equal(got, want.astype(np.uint32)), desc
