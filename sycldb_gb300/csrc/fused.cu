@@ -1278,15 +1278,15 @@ __device__ __forceinline__ void run_steps1(const Launch &L, RowT &R, const uint3
 // be converged.
 // Writes the first-writer's key values of slot sl: key(std::integral_constant
 // <int, q>) gives key q.
-template <class KeyFn, int... KK>
-__device__ __forceinline__ void write_keys(const Launch &L, int nk, int64_t sl, KeyFn &key,
+template <class LaunchT, class KeyFn, int... KK>
+__device__ __forceinline__ void write_keys(const LaunchT &L, int nk, int64_t sl, KeyFn &key,
                                            std::integer_sequence<int, KK...>)
 {
     ((KK < nk ? (void)(L.out_keys[KK][sl] = key(std::integral_constant<int, KK>{})) : (void)0), ...);
 }
 
-template <class KeyFn>
-__device__ __forceinline__ void group_row(const Launch &L, uint32_t *s_key, unsigned long long *s_sum, bool direct,
+template <class LaunchT, class KeyFn>
+__device__ __forceinline__ void group_row(const LaunchT &L, uint32_t *s_key, unsigned long long *s_sum, bool direct,
                                           bool row, uint32_t h, int32_t value, int nk, KeyFn key)
 {
     const int64_t sl = row ? sdb::group_slot(h, L.P) : 0;
@@ -1336,7 +1336,8 @@ __device__ __forceinline__ void group_table_reset(uint32_t *s_key, unsigned long
 
 // Packs the chain's semi-join table into the shared-memory bitmap: word w
 // holds entries 32w .. 32w + 31.
-__device__ __forceinline__ void stage_bitmap(const Launch &L, uint32_t *s_bits)
+template <class LaunchT>
+__device__ __forceinline__ void stage_bitmap(const LaunchT &L, uint32_t *s_bits)
 {
     if (!L.bitmap_ht) return;
     const uint32_t words = (L.bitmap_len + 31) / 32;
@@ -1755,8 +1756,8 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
 // Flushes a block's partials of one chain into its global outputs: one
 // 64-bit atomic per block for SUM, one per touched slot for group-by.  The
 // caller synchronises the block before and (to reuse the table) after.
-template <int TERM>
-__device__ __forceinline__ void block_flush(const Launch &L, uint32_t *s_key, unsigned long long *s_sum,
+template <int TERM, class LaunchT>
+__device__ __forceinline__ void block_flush(const LaunchT &L, uint32_t *s_key, unsigned long long *s_sum,
                                             uint64_t *s_part, uint64_t &acc)
 {
     if (TERM == T_SUM) {
@@ -2629,6 +2630,52 @@ bool pairable(const Launch &A, const Launch &B, int term_a, int term_b)
 
 }  // namespace dense
 
+// A selection of a value against literals as an interval test (the fields of
+// RangeTest that hold it): SELECT by cmp_op against v, SEARCH_RANGE lo .. hi,
+// SEARCH_POINTS lo or hi.  The test holds for exactly the values the
+// comparison holds for.  False for another op or an unknown comparison.
+bool range_test(int kind, int cmp_op, int32_t v, int32_t lo, int32_t hi, RangeTest &t)
+{
+    constexpr int32_t kMin = INT32_MIN, kMax = INT32_MAX;
+    bool never = false;
+    if (kind == SDB_OP_SELECT) {
+        switch (cmp_op) {
+        case SDB_EQ: t.lo = v; t.span = 0; break;
+        case SDB_NE: t.lo = v; t.span = 0; t.neg = 1; break;
+        case SDB_LT:
+            if (v == kMin) never = true;
+            else { t.lo = kMin; t.span = (uint32_t)(v - 1) - (uint32_t)kMin; }
+            break;
+        case SDB_LE: t.lo = kMin; t.span = (uint32_t)v - (uint32_t)kMin; break;
+        case SDB_GT:
+            if (v == kMax) never = true;
+            else { t.lo = v + 1; t.span = (uint32_t)kMax - (uint32_t)(v + 1); }
+            break;
+        case SDB_GE: t.lo = v; t.span = (uint32_t)kMax - (uint32_t)v; break;
+        default: return false;
+        }
+        t.lo2 = t.lo;
+        t.span2 = t.span;
+    } else if (kind == SDB_OP_SEARCH_RANGE) {
+        if (lo > hi) never = true;
+        else { t.lo = t.lo2 = lo; t.span = t.span2 = (uint32_t)hi - (uint32_t)lo; }
+    } else if (kind == SDB_OP_SEARCH_POINTS) {
+        t.lo = lo;
+        t.lo2 = hi;
+        t.span = t.span2 = 0;
+    } else {
+        return false;
+    }
+    if (never) {  // no value: the complement of every value
+        t.lo = t.lo2 = kMin;
+        t.span = t.span2 = 0xffffffffu;
+        t.neg = 1;
+    }
+    return true;
+}
+
+#include "sieve.cuh"
+
 // Tuning table: variant per (terminal, register class, kind of the first op,
 // log2 rows bucket); -1 = default.  Set by sdb_chain_tune_set(_op) (the
 // autotuner persists its choices and loads them at start-up).  The first op
@@ -2697,13 +2744,11 @@ bool operand_ok(const sdb_operand &o, int &nregs, bool &vec, const char **why)
     return true;
 }
 
-// A build chain's ops as interval tests (RangeTest), or -1 when some op is
-// not a selection of a column against literals (or uses a code the general
-// pass treats specially) or there are more than kRangeTests.  Each test holds
-// for exactly the values the op's comparison holds for.
+// A build chain's ops as interval tests, or -1 when some op is not a
+// selection of a column against literals (or uses a code the general pass
+// treats specially) or there are more than kRangeTests.
 int range_tests(const sdb_chain_desc &c, RangeTest *out)
 {
-    constexpr int32_t kMin = INT32_MIN, kMax = INT32_MAX;
     if (c.n_ops > kRangeTests || c.n >= (1ull << 32) - 4096) return -1;
     if ((c.build_key.kind != SDB_SRC_COL && c.build_key.kind != SDB_SRC_LIT) ||
         (c.terminal == SDB_TERM_BUILD_KV && c.build_val.kind != SDB_SRC_COL && c.build_val.kind != SDB_SRC_LIT))
@@ -2712,44 +2757,10 @@ int range_tests(const sdb_chain_desc &c, RangeTest *out)
         const sdb_chain_op &o = c.ops[i];
         RangeTest t{};
         if (o.a.kind != SDB_SRC_COL || o.logic_op < SDB_NONE || o.logic_op > SDB_OR) return -1;
+        if (o.kind == SDB_OP_SELECT && o.b.kind != SDB_SRC_LIT) return -1;
+        if (!range_test(o.kind, o.cmp_op, o.b.lit, o.lo, o.hi, t)) return -1;
         t.col = o.a.col;
         t.logic = o.logic_op;
-        bool never = false;
-        if (o.kind == SDB_OP_SELECT) {
-            if (o.b.kind != SDB_SRC_LIT) return -1;
-            const int32_t v = o.b.lit;
-            switch (o.cmp_op) {
-            case SDB_EQ: t.lo = v; t.span = 0; break;
-            case SDB_NE: t.lo = v; t.span = 0; t.neg = 1; break;
-            case SDB_LT:
-                if (v == kMin) never = true;
-                else { t.lo = kMin; t.span = (uint32_t)(v - 1) - (uint32_t)kMin; }
-                break;
-            case SDB_LE: t.lo = kMin; t.span = (uint32_t)v - (uint32_t)kMin; break;
-            case SDB_GT:
-                if (v == kMax) never = true;
-                else { t.lo = v + 1; t.span = (uint32_t)kMax - (uint32_t)(v + 1); }
-                break;
-            case SDB_GE: t.lo = v; t.span = (uint32_t)kMax - (uint32_t)v; break;
-            default: return -1;
-            }
-            t.lo2 = t.lo;
-            t.span2 = t.span;
-        } else if (o.kind == SDB_OP_SEARCH_RANGE) {
-            if (o.lo > o.hi) never = true;
-            else { t.lo = t.lo2 = o.lo; t.span = t.span2 = (uint32_t)o.hi - (uint32_t)o.lo; }
-        } else if (o.kind == SDB_OP_SEARCH_POINTS) {
-            t.lo = o.lo;
-            t.lo2 = o.hi;
-            t.span = t.span2 = 0;
-        } else {
-            return -1;
-        }
-        if (never) {  // no value: the complement of every value
-            t.lo = t.lo2 = kMin;
-            t.span = t.span2 = 0xffffffffu;
-            t.neg = 1;
-        }
         out[i] = t;
     }
     return c.n_ops;
@@ -2895,6 +2906,8 @@ static int fused_chain_impl(const sdb_chain_desc *chain, int variant, sdb_stream
         const int st2 = dense::dispatch(L, nregs, term, variant != kDenseVariant, variant_stages(variant),
                                         variant_carry(variant), s);
         if (st2 != SDB_ERR_UNSUPPORTED) return st2;
+        const int st3 = sieve::dispatch(L, nregs, term, s);
+        if (st3 != SDB_ERR_UNSUPPORTED) return st3;
         variant = default_variant(nregs);
     }
     switch (term) {
