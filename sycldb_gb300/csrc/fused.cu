@@ -13,7 +13,7 @@
 //   - intermediate columns (join values, projections) live in registers and
 //     are stored only when the caller asks for them (out_col);
 //   - group-by partial sums are privatised in shared memory per block
-//     (64-bit shared atomics) and flushed once per touched slot; the first
+//     (32-bit shared atomics, carry by hand) and flushed once per touched slot; the first
 //     block to touch a slot runs the reference's first-writer exchange
 //     (kernels/aggregation.hpp:329-333) on the global occupancy word.
 // Grids are persistent: (#SMs x resident blocks), grid-stride over 4-row
@@ -292,17 +292,39 @@ __device__ __forceinline__ void run_ops(const LC &Lc, Tile<NREGS, ITEMS> &T)
     }
 }
 
-// Block-private group-by partials: a shared-memory table of kCap entries
-// (slot id + 64-bit sum, 24 KB).  Slots index it directly when P <= kCap;
-// otherwise it is an open-addressing table (bounded linear probing) and a
-// row that finds no entry goes straight to the global arrays.
+// Block-private group-by partials: a shared-memory table of CAP entries
+// (slot id, then the 64-bit sums as CAP low words and CAP high words).  Slots
+// index it directly when P <= CAP; otherwise it is an open-addressing table
+// (bounded linear probing) and a row that finds no entry goes straight to the
+// global arrays.
 constexpr uint32_t kCap = 2048;
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;
 constexpr int kMaxProbe = 16;
 
+// s_sum[h] += v (sign-extended) with the shared-memory atomics the SM has
+// natively, the 32-bit ones: the low word's add returns what it held, so its
+// carry and the sign go into the high word, which most adds do not touch.
+// Measured, cycles of an SM per warp with 1 / 2 / 7 / 50 / 280 groups: 33 / 19 /
+// 9 / 9 / 9; 64-bit shared atomics (a compare-and-swap loop) 786 / 451 / 152 /
+// 50 / 28; lanes of one slot summed first (__match_any_sync and two
+// __reduce_add_sync, which run once per distinct slot) 23 / 31 / 77 / 115 / 85.
+template <uint32_t CAP>
+__device__ __forceinline__ void smem_sum_add(uint32_t *s_sum, uint32_t h, int32_t v)
+{
+    const uint32_t old = atomicAdd(&s_sum[h], (uint32_t)v);
+    const uint32_t hi = (uint32_t)(old + (uint32_t)v < old) + (uint32_t)(v >> 31);
+    if (hi) atomicAdd(&s_sum[CAP + h], hi);
+}
+
+template <uint32_t CAP>
+__device__ __forceinline__ unsigned long long smem_sum(const uint32_t *s_sum, uint32_t h)
+{
+    return (unsigned long long)s_sum[h] | ((unsigned long long)s_sum[CAP + h] << 32);
+}
+
 template <uint32_t CAP = kCap>
-__device__ __forceinline__ bool smem_group_add(uint32_t *s_key, unsigned long long *s_sum, uint32_t slot,
-                                               unsigned long long v, bool direct, bool &first)
+__device__ __forceinline__ bool smem_group_add(uint32_t *s_key, uint32_t *s_sum, uint32_t slot, int32_t v, bool direct,
+                                               bool &first)
 {
     static_assert((CAP & (CAP - 1)) == 0, "table size must be a power of two");
     uint32_t h = direct ? slot : ((slot * 2654435761u) >> (32 - __builtin_ctz(CAP)));
@@ -313,13 +335,13 @@ __device__ __forceinline__ bool smem_group_add(uint32_t *s_key, unsigned long lo
             k = atomicCAS(&s_key[h], kEmpty, slot);
             if (k == kEmpty) {
                 first = true;
-                atomicAdd(&s_sum[h], v);
+                smem_sum_add<CAP>(s_sum, h, v);
                 return true;
             }
         }
         if (k == slot) {
             first = false;
-            atomicAdd(&s_sum[h], v);
+            smem_sum_add<CAP>(s_sum, h, v);
             return true;
         }
         h = (h + 1) & (CAP - 1);
@@ -504,12 +526,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks_of(ITEMS)) k_chain(const 
 {
     const sdb_chain_desc &d = L.d;
     __shared__ uint32_t s_key[TERM == T_GROUP ? kCap : 1];
-    __shared__ unsigned long long s_sum[TERM == T_GROUP ? kCap : 1];
+    __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kCap : 1];
     const bool direct = d.P <= kCap;
     if (TERM == T_GROUP) {
         for (uint32_t i = threadIdx.x; i < kCap; i += blockDim.x) {
             s_key[i] = kEmpty;
-            s_sum[i] = 0;
+            s_sum[i] = s_sum[kCap + i] = 0;
         }
         __syncthreads();
     }
@@ -571,13 +593,12 @@ __global__ void __launch_bounds__(kThreads, min_blocks_of(ITEMS)) k_chain(const 
                     atomicAdd(&g_errors, 1ull);
                     continue;
                 }
-                const unsigned long long val = (unsigned long long)sdb::widen(v[k]);
                 bool first = false;
-                if (smem_group_add(s_key, s_sum, (uint32_t)s, val, direct, first)) {
+                if (smem_group_add(s_key, s_sum, (uint32_t)s, v[k], direct, first)) {
                     if (first) first = atomicExch(&d.occ[s], 1u) == 0u;
                 } else {
                     first = d.occ[s] == 0u && atomicExch(&d.occ[s], 1u) == 0u;
-                    atomicAdd(reinterpret_cast<unsigned long long *>(&d.out_sum[s]), val);
+                    atomicAdd(reinterpret_cast<unsigned long long *>(&d.out_sum[s]), (unsigned long long)sdb::widen(v[k]));
                 }
                 if (first) {
 #pragma unroll
@@ -603,7 +624,7 @@ __global__ void __launch_bounds__(kThreads, min_blocks_of(ITEMS)) k_chain(const 
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < kCap; i += blockDim.x) {
             const uint32_t k = s_key[i];
-            if (k != kEmpty) atomicAdd(reinterpret_cast<unsigned long long *>(&d.out_sum[k]), s_sum[i]);
+            if (k != kEmpty) atomicAdd(reinterpret_cast<unsigned long long *>(&d.out_sum[k]), smem_sum<kCap>(s_sum, i));
         }
     }
 }
@@ -1270,12 +1291,6 @@ __device__ __forceinline__ void run_steps1(const Launch &L, RowT &R, const uint3
      ...);
 }
 
-// Adds the lane's row (when `row`) to the group-by (block table first, global
-// on overflow) and runs the first-writer exchange; key(std::integral_constant
-// <int, q>) gives the row's key q, nk the number of keys.  All 32 lanes of the warp call it (with row false where the
-// lane holds none): the lanes that take part in the warp aggregation are
-// named by a ballot over the full warp, never by the lanes that happen to
-// be converged.
 // Writes the first-writer's key values of slot sl: key(std::integral_constant
 // <int, q>) gives key q.
 template <class LaunchT, class KeyFn, int... KK>
@@ -1285,33 +1300,24 @@ __device__ __forceinline__ void write_keys(const LaunchT &L, int nk, int64_t sl,
     ((KK < nk ? (void)(L.out_keys[KK][sl] = key(std::integral_constant<int, KK>{})) : (void)0), ...);
 }
 
+// Adds a row to the group-by (block table first, global on overflow) and runs
+// the first-writer exchange; key(std::integral_constant<int, q>) gives the
+// row's key q, nk the number of keys.
 template <class LaunchT, class KeyFn>
-__device__ __forceinline__ void group_row(const LaunchT &L, uint32_t *s_key, unsigned long long *s_sum, bool direct,
-                                          bool row, uint32_t h, int32_t value, int nk, KeyFn key)
+__device__ __forceinline__ void group_row(const LaunchT &L, uint32_t *s_key, uint32_t *s_sum, bool direct, uint32_t h,
+                                          int32_t value, int nk, KeyFn key)
 {
-    const int64_t sl = row ? sdb::group_slot(h, L.P) : 0;
-    const bool bad = row && (sl < 0 || (uint64_t)sl >= L.P);
-    if (bad) atomicAdd(&g_errors, 1ull);
-    const bool go = row && !bad;
-    const unsigned mask = __ballot_sync(0xffffffffu, go);
-    if (!go) return;
-    unsigned long long val = (unsigned long long)sdb::widen(value);
-    // warp aggregation: lanes here with the same slot sum their values (exactly:
-    // 16-bit halves reduced in 32 bits, then recombined in 64) and only the
-    // lowest of them updates the table
-    const unsigned peers = __match_any_sync(mask, (unsigned)sl);
-    if (__popc(peers) > 1) {
-        const uint32_t lo = __reduce_add_sync(peers, (uint32_t)value & 0xffffu);
-        const int32_t hi = (int32_t)__reduce_add_sync(peers, (uint32_t)(value >> 16));
-        if ((threadIdx.x & 31u) != (unsigned)(__ffs(peers) - 1)) return;
-        val = (unsigned long long)((int64_t)hi * 65536 + (int64_t)lo);
+    const int64_t sl = sdb::group_slot(h, L.P);
+    if (sl < 0 || (uint64_t)sl >= L.P) {
+        atomicAdd(&g_errors, 1ull);
+        return;
     }
     bool first = false;
-    if (smem_group_add<kDenseCap>(s_key, s_sum, (uint32_t)sl, val, direct, first)) {
+    if (smem_group_add<kDenseCap>(s_key, s_sum, (uint32_t)sl, value, direct, first)) {
         if (first) first = atomicExch(&L.occ[sl], 1u) == 0u;
     } else {
         first = L.occ[sl] == 0u && atomicExch(&L.occ[sl], 1u) == 0u;
-        atomicAdd(reinterpret_cast<unsigned long long *>(&L.out_sum[sl]), val);
+        atomicAdd(reinterpret_cast<unsigned long long *>(&L.out_sum[sl]), (unsigned long long)sdb::widen(value));
     }
     if (first) write_keys(L, nk, sl, key, std::make_integer_sequence<int, SDB_CHAIN_MAX_KEYS>{});
 }
@@ -1325,12 +1331,12 @@ __host__ __device__ constexpr int dense_min_blocks() { return CARRY == 3 ? 5 : (
 // ---- pieces shared by the single-chain pass and the batched pass ----------
 
 template <int TERM>
-__device__ __forceinline__ void group_table_reset(uint32_t *s_key, unsigned long long *s_sum)
+__device__ __forceinline__ void group_table_reset(uint32_t *s_key, uint32_t *s_sum)
 {
     if (TERM == T_GROUP)
         for (uint32_t i = threadIdx.x; i < kDenseCap; i += blockDim.x) {
             s_key[i] = kEmpty;
-            s_sum[i] = 0;
+            s_sum[i] = s_sum[kDenseCap + i] = 0;
         }
 }
 
@@ -1417,26 +1423,23 @@ __device__ __forceinline__ uint32_t key_hash(const Launch &L, const RowT &R, int
 }
 
 template <int TERM, class B, class RowT>
-__device__ __forceinline__ void finish_row(const Launch &L, RowT &R, uint32_t *s_key, unsigned long long *s_sum,
+__device__ __forceinline__ void finish_row(const Launch &L, RowT &R, uint32_t *s_key, uint32_t *s_sum,
                                            bool direct, uint64_t &acc)
 {
     if (TERM == T_SUM) {
         if (R.live) acc += sdb::widen(fetch1c<B::value()>(L.value, R));
-    } else if (TERM == T_GROUP) {
-        // every lane of the warp reaches group_row (its warp aggregation
-        // needs the whole warp); values of a lane without a live row are
-        // read from its registers or staged rows and not used
+    } else if (TERM == T_GROUP && R.live) {
         const int nk = B::n_keys() == kAny ? L.n_keys : B::n_keys();
         const uint32_t h = key_hash<B>(L, R, nk, std::make_integer_sequence<int, SDB_CHAIN_MAX_KEYS>{});
         auto key = [&R, &L](auto q) { return fetch1c<B::key(decltype(q)::value)>(L.keys[decltype(q)::value], R); };
-        group_row(L, s_key, s_sum, direct, R.live, h, fetch1c<B::value()>(L.value, R), nk, key);
+        group_row(L, s_key, s_sum, direct, h, fetch1c<B::value()>(L.value, R), nk, key);
     }
 }
 
 // The ops from SPLIT on and the terminal, for one row held by one lane.
 template <int TERM, class B, int NREGS, int SPLIT, int... KS, class RowT>
 __device__ __forceinline__ void sparse_row(const Launch &L, RowT &R, const uint32_t *s_bits, uint32_t *s_key,
-                                           unsigned long long *s_sum, bool direct, uint64_t &acc)
+                                           uint32_t *s_sum, bool direct, uint64_t &acc)
 {
     constexpr int N = sizeof...(KS);
 #pragma unroll
@@ -1486,7 +1489,7 @@ __device__ __forceinline__ VRow<NREGS> take_row(const VRow<NREGS> &R, const uint
 // slots of each live row from its row number.
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_run(const Launch &L, VRow<NREGS> &F, const uint32_t *s_bits, uint32_t *s_key,
-                                           unsigned long long *s_sum, bool direct, uint64_t &acc)
+                                           uint32_t *s_sum, bool direct, uint64_t &acc)
 {
     constexpr int N = sizeof...(KS);
     if constexpr (CARRY == 3) {
@@ -1506,7 +1509,7 @@ __device__ __forceinline__ void level2_run(const Launch &L, VRow<NREGS> &F, cons
 // level-2 rows and runs the remaining ops whenever 32 are pending.
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_push(const Launch &L, const VRow<NREGS> &R, Level2<NREGS> &Q,
-                                            const uint32_t *s_bits, uint32_t *s_key, unsigned long long *s_sum,
+                                            const uint32_t *s_bits, uint32_t *s_key, uint32_t *s_sum,
                                             bool direct, uint64_t &acc)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -1548,7 +1551,7 @@ __host__ __device__ constexpr bool use_level2(int carry)
 // The first row-per-lane op and then the second level, for one group.
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_group(const Launch &L, VRow<NREGS> &R, Level2<NREGS> &Q, const uint32_t *s_bits,
-                                             uint32_t *s_key, unsigned long long *s_sum, bool direct, uint64_t &acc)
+                                             uint32_t *s_key, uint32_t *s_sum, bool direct, uint64_t &acc)
 {
     constexpr int kinds[] = {KS...};
 #pragma unroll
@@ -1560,7 +1563,7 @@ __device__ __forceinline__ void level2_group(const Launch &L, VRow<NREGS> &R, Le
 // Runs whatever the warp still holds (at the end of a block's rows of a chain).
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void drain_carry(const Launch &L, uint32_t &carry, const int4 &ce, Level2<NREGS> &Q,
-                                            const uint32_t *s_bits, uint32_t *s_key, unsigned long long *s_sum,
+                                            const uint32_t *s_bits, uint32_t *s_key, uint32_t *s_sum,
                                             bool direct, uint64_t &acc)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -1610,7 +1613,7 @@ __device__ __forceinline__ int32_t tail_value(const Launch &L, const int32_t *ws
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of<CARRY>()> &S, const int4 *s_buf, int st,
                                           uint64_t tile,
-                                          uint8_t *s_list, uint32_t *s_key, unsigned long long *s_sum,
+                                          uint8_t *s_list, uint32_t *s_key, uint32_t *s_sum,
                                           const uint32_t *s_bits, bool direct, uint64_t &acc, uint32_t &carry,
                                           int4 &ce, Level2<NREGS> &Q)
 {
@@ -1727,10 +1730,7 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
 #pragma unroll
             for (int k = 0; k < kItems; k++)
                 if ((S.live >> k) & 1u) acc += sdb::widen(v[k]);
-        } else if (TERM == T_GROUP && __any_sync(0xffffffffu, S.live != 0)) {
-            // the whole warp runs the group-by of its items (group_row's
-            // warp aggregation needs every lane); staged values of dead or
-            // missing rows are read and not used
+        } else if (TERM == T_GROUP && S.live) {
             int32_t v[kItems];
             fetch4(L.value, S, v);
             uint32_t h[kItems] = {};
@@ -1744,7 +1744,7 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
                 }
 #pragma unroll
             for (int k = 0; k < kItems; k++)
-                group_row(L, s_key, s_sum, direct, ((S.live >> k) & 1u) != 0, h[k], v[k], L.n_keys, [&](auto q) {
+                if ((S.live >> k) & 1u) group_row(L, s_key, s_sum, direct, h[k], v[k], L.n_keys, [&](auto q) {
                     int32_t kv[kItems];
                     fetch4(L.keys[decltype(q)::value], S, kv);
                     return kv[k];
@@ -1757,7 +1757,7 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
 // 64-bit atomic per block for SUM, one per touched slot for group-by.  The
 // caller synchronises the block before and (to reuse the table) after.
 template <int TERM, class LaunchT>
-__device__ __forceinline__ void block_flush(const LaunchT &L, uint32_t *s_key, unsigned long long *s_sum,
+__device__ __forceinline__ void block_flush(const LaunchT &L, uint32_t *s_key, uint32_t *s_sum,
                                             uint64_t *s_part, uint64_t &acc)
 {
     if (TERM == T_SUM) {
@@ -1775,7 +1775,7 @@ __device__ __forceinline__ void block_flush(const LaunchT &L, uint32_t *s_key, u
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < kDenseCap; i += blockDim.x) {
             const uint32_t k = s_key[i];
-            if (k != kEmpty) atomicAdd(reinterpret_cast<unsigned long long *>(&L.out_sum[k]), s_sum[i]);
+            if (k != kEmpty) atomicAdd(reinterpret_cast<unsigned long long *>(&L.out_sum[k]), smem_sum<kDenseCap>(s_sum, i));
         }
     }
 }
@@ -1789,7 +1789,7 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>()) k
     constexpr int SS = stage_slots<CARRY>();
     extern __shared__ int4 s_buf[];  // [kStages][SS][kThreads][kQ], then the semi-join bitmap
     __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
-    __shared__ unsigned long long s_sum[TERM == T_GROUP ? kDenseCap : 1];
+    __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kDenseCap : 1];
     __shared__ uint8_t s_list[kCompact ? kThreads * kItems : 1];  // per warp: 32 x kItems row offsets
     __shared__ uint64_t s_part[kThreads / 32];
     __shared__ uint8_t s_l2src[CARRY >= 2 ? kThreads : 1];
@@ -1857,7 +1857,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_dense_pair(const __grid_constan
     constexpr int SS = stage_slots<CARRY>();
     extern __shared__ int4 s_buf[];  // [kStages][SS][kThreads][kQ], then the chains' bitmaps
     __shared__ uint32_t s_key[kPair][TERM == T_GROUP ? kDenseCap : 1];
-    __shared__ unsigned long long s_sum[kPair][TERM == T_GROUP ? kDenseCap : 1];
+    __shared__ uint32_t s_sum[kPair][TERM == T_GROUP ? 2 * kDenseCap : 1];
     __shared__ uint8_t s_list[kCompact ? kThreads * kItems : 1];  // reused by the chains in turn
     __shared__ uint64_t s_part[kThreads / 32];
     __shared__ uint8_t s_l2src[kPair][kThreads];
@@ -1952,7 +1952,7 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>())
     constexpr uint64_t kTile = (uint64_t)kThreads * kItems;
     extern __shared__ int4 s_buf[];
     __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
-    __shared__ unsigned long long s_sum[TERM == T_GROUP ? kDenseCap : 1];
+    __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kDenseCap : 1];
     __shared__ uint8_t s_list[kCompact ? kThreads * kItems : 1];
     __shared__ uint64_t s_part[kThreads / 32];
     __shared__ Launch s_L;

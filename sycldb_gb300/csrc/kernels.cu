@@ -355,24 +355,30 @@ __device__ __forceinline__ void claim_keys(const GroupArgs &a, int64_t h, uint64
 }
 
 // Shared-memory privatised slot sums; a block's first touch of a slot also
-// runs the global first-writer exchange; sums flush once per touched slot.
+// runs the global first-writer exchange; sums flush once per touched slot.  A
+// slot's 64-bit sum is a low and a high word (s_lo[h], s_lo[P + h]) added with
+// 32-bit atomics, the low word's carry taken from the value its add returns:
+// 64-bit shared atomics are compare-and-swap loops (28 cycles of an SM per
+// warp over 280 slots, 450 over two; 9 and 19 this way).
 // One flagged row's slot update (K8): the first writer of a slot stores its
 // keys, the value goes into the slot's sum.
 template <bool SMEM>
-__device__ __forceinline__ void group_row(const GroupArgs &a, uint64_t r, uint64_t *s_sum, uint32_t *s_occ)
+__device__ __forceinline__ void group_row(const GroupArgs &a, uint64_t r, uint32_t *s_lo, uint32_t *s_occ)
 {
     const int64_t h = row_slot(a, r);
     if (h < 0 || (uint64_t)h >= a.P) {
         atomicAdd(&g_errors, 1ull);
         return;
     }
-    const unsigned long long v = (unsigned long long)sdb::widen(a.val[r]);
+    const int32_t v = a.val[r];
     if (SMEM) {
-        if (atomicExch(&s_occ[h], 1u) == 0u) claim_keys(a, h, r);
-        atomicAdd(reinterpret_cast<unsigned long long *>(&s_sum[h]), v);
+        if (s_occ[h] == 0u && atomicExch(&s_occ[h], 1u) == 0u) claim_keys(a, h, r);
+        const uint32_t old = atomicAdd(&s_lo[h], (uint32_t)v);
+        const uint32_t hi = (uint32_t)(old + (uint32_t)v < old) + (uint32_t)(v >> 31);
+        if (hi) atomicAdd(&s_lo[a.P + h], hi);
     } else {
         if (a.occ[h] == 0u) claim_keys(a, h, r);
-        atomicAdd(reinterpret_cast<unsigned long long *>(&a.out_sum[h]), v);
+        atomicAdd(reinterpret_cast<unsigned long long *>(&a.out_sum[h]), (unsigned long long)sdb::widen(v));
     }
 }
 
@@ -386,13 +392,13 @@ constexpr int kGroupList = 32 * 16;  // a warp's rows per iteration
 template <bool SMEM, bool VEC>
 __global__ void __launch_bounds__(kThreads) k_groupby(const GroupArgs a)
 {
-    extern __shared__ uint64_t s_sum[];
-    uint32_t *s_occ = reinterpret_cast<uint32_t *>(s_sum + (SMEM ? a.P : 0));
-    uint32_t *s_list = s_occ + (SMEM ? ((a.P + 1) & ~1ull) : 0);  // 8-byte aligned after the table
+    extern __shared__ uint32_t s_lo[];  // P low words, P high words, P occupancy words, the lists
+    uint32_t *s_occ = s_lo + (SMEM ? 2 * a.P : 0);
+    uint32_t *s_list = s_occ + (SMEM ? a.P : 0);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t *list = s_list + warp * kGroupList;
     if (SMEM) {
-        for (uint64_t i = threadIdx.x; i < a.P; i += blockDim.x) { s_sum[i] = 0; s_occ[i] = 0; }
+        for (uint64_t i = threadIdx.x; i < 3 * a.P; i += blockDim.x) s_lo[i] = 0;
         __syncthreads();
     }
     const uint64_t groups = (a.n + 15) / 16;
@@ -432,13 +438,15 @@ __global__ void __launch_bounds__(kThreads) k_groupby(const GroupArgs a)
         }
         __syncwarp();
         const uint64_t base = c * 32 * 16;
-        for (uint32_t i = lane; i < total; i += 32) group_row<SMEM>(a, base + list[i], s_sum, s_occ);
+        for (uint32_t i = lane; i < total; i += 32) group_row<SMEM>(a, base + list[i], s_lo, s_occ);
         __syncwarp();
     }
     if (SMEM) {
         __syncthreads();
         for (uint64_t i = threadIdx.x; i < a.P; i += blockDim.x)
-            if (s_occ[i]) atomicAdd(reinterpret_cast<unsigned long long *>(&a.out_sum[i]), (unsigned long long)s_sum[i]);
+            if (s_occ[i])
+                atomicAdd(reinterpret_cast<unsigned long long *>(&a.out_sum[i]),
+                          (unsigned long long)s_lo[i] | ((unsigned long long)s_lo[a.P + i] << 32));
     }
 }
 
@@ -1039,10 +1047,9 @@ int sdb_groupby_sum(const int32_t *const *keys, const int32_t *mins, const int32
     a.g = g; a.val = val; a.flags = flags; a.n = n; a.P = P; a.out_sum = out_sum; a.occ = occ;
     if (n == 0) return SDB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    // the slot table (P <= 8192: 12 B per slot, the occupancy words padded to
-    // 8 bytes) and every warp's row list
+    // the slot table (P <= 8192: 12 B per slot) and every warp's row list
     const size_t list_bytes = (size_t)(kThreads / 32) * kGroupList * sizeof(uint32_t);
-    const size_t smem = (P <= 8192 ? (size_t)P * sizeof(uint64_t) + ((P + 1) & ~1ull) * sizeof(uint32_t) : 0) + list_bytes;
+    const size_t smem = (P <= 8192 ? (size_t)P * 3 * sizeof(uint32_t) : 0) + list_bytes;
     const uint64_t groups = (n + 15) / 16;
     const bool vec = sdb::aligned(flags, 16);
     static const bool attr_set = [] {  // once, thread-safe

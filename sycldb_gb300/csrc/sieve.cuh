@@ -267,34 +267,33 @@ __device__ __forceinline__ void row_op(const Op &op, Row<NREGS> &R, const uint32
     }
 }
 
-// The terminal for one row per lane (every lane of the warp calls it).
+// The terminal for one row per lane.
 template <int TERM, int NREGS>
-__device__ __forceinline__ void finish(const Launch &L, const Row<NREGS> &R, uint32_t *s_key, unsigned long long *s_sum,
-                                       bool direct, uint64_t &acc)
+__device__ __forceinline__ void finish(const Launch &L, const Row<NREGS> &R, uint32_t *s_key, uint32_t *s_sum, bool direct,
+                                       uint64_t &acc)
 {
+    if (!R.live) return;
+    const int32_t value = get(L.value, R);
     if (TERM == T_SUM) {
-        if (R.live) acc += sdb::widen(get(L.value, R));
+        acc += sdb::widen(value);
     } else {
         static_assert(SDB_CHAIN_MAX_KEYS == 4, "four keys by name");
-        int32_t value = 0, k0 = 0, k1 = 0, k2 = 0, k3 = 0;
+        int32_t k0 = 0, k1 = 0, k2 = 0, k3 = 0;
         uint32_t h = 0;
-        if (R.live) {
-            value = get(L.value, R);
-            auto add = [&](int q, int32_t &k) {
-                if (q >= L.n_keys) return;
-                k = get(L.keys[q], R);
-                h += ((uint32_t)k - (uint32_t)L.key_min[q]) * L.mults[q];
-            };
-            add(0, k0);
-            add(1, k1);
-            add(2, k2);
-            add(3, k3);
-        }
+        auto add = [&](int q, int32_t &k) {
+            if (q >= L.n_keys) return;
+            k = get(L.keys[q], R);
+            h += ((uint32_t)k - (uint32_t)L.key_min[q]) * L.mults[q];
+        };
+        add(0, k0);
+        add(1, k1);
+        add(2, k2);
+        add(3, k3);
         auto key_of = [k0, k1, k2, k3](auto q) {
             constexpr int i = decltype(q)::value;
             return i == 0 ? k0 : (i == 1 ? k1 : (i == 2 ? k2 : k3));
         };
-        dense::group_row(L, s_key, s_sum, direct, R.live, h, value, L.n_keys, key_of);
+        dense::group_row(L, s_key, s_sum, direct, h, value, L.n_keys, key_of);
     }
 }
 
@@ -303,7 +302,7 @@ __global__ void __launch_bounds__(kThreads, TERM == T_FLAGS ? 6 : 5) k_sieve(con
 {
     extern __shared__ int4 s_buf[];  // [kStages][kStaged][kThreads][kQ], then the queues and the bitmap
     __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
-    __shared__ unsigned long long s_sum[TERM == T_GROUP ? kDenseCap : 1];
+    __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kDenseCap : 1];
     __shared__ uint8_t s_list[TERM == T_FLAGS ? 1 : kThreads * kItems];  // per warp: offsets of its surviving rows
     __shared__ uint64_t s_part[kWarps];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
