@@ -50,6 +50,8 @@
 #include "sycldb_gpu.h"
 
 int sdb_set_error(int status, const char *fmt, ...);
+int sdb_compact_gather_large(const void *flags, bool occ, uint64_t n, int ncols, const void *const *src, const int *wide,
+                             void *const *dst, uint32_t *count, void *scratch, cudaStream_t s);  // kernels.cu
 
 namespace sdb {
 
@@ -2037,71 +2039,44 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
         o.cap = cnt;
         MemoryManager &R = E.rmm ? *E.rmm : E.mm;
         const uint8_t *fl0 = fin.flags + sg[s].first;
-        if (cnt <= 65536 && cols.size() <= 8) {  // small result: compaction and gathers in one launch
-            uint32_t *count = R.alloc<uint32_t>(1);
-            o.count = count;
-            std::vector<const void *> src;
-            std::vector<void *> dst;
-            std::vector<int> wide;
-            for (Column *c : cols) {
-                const Segment &seg = c->segments[s];
-                if (c->is_aggregate_result) {
-                    src.push_back(seg.agg);
-                    dst.push_back(R.alloc<uint64_t>(cnt));
-                    wide.push_back(1);
-                } else {
-                    src.push_back(seg.data);
-                    dst.push_back(R.alloc<int32_t>(cnt));
-                    wide.push_back(0);
-                }
-            }
-            o.dev = dst;
-            auto oc = E.from_occ.find(fl0);
-            if (oc != E.from_occ.end()) {  // a group-by result: straight from its occupancy words
-                const uint32_t *occ = oc->second.first;
-                E.dev("compact_gather", [occ, cnt, src, wide, dst, count](cudaStream_t st) {
-                    return sdb_compact_gather_occ(occ, cnt, (int)src.size(), src.data(), wide.data(), dst.data(), count,
-                                                  (sdb_stream_t)st);
-                });
-            } else {
-                E.ensure_filled(fl0);
-                E.dev("compact_gather", [fl0, cnt, src, wide, dst, count](cudaStream_t st) {
-                    return sdb_compact_gather(fl0, cnt, (int)src.size(), src.data(), wide.data(), dst.data(), count,
-                                              (sdb_stream_t)st);
-                });
-            }
-            pr.segs.push_back(o);
-            continue;
-        }
-        int32_t *ids = E.mm.alloc<int32_t>(cnt);
         uint32_t *count = R.alloc<uint32_t>(1);
         o.count = count;
-        size_t sb = sdb_compact_scratch_bytes(cnt);
-        void *scratch = E.mm.alloc<uint8_t>(sb);
-        const uint8_t *fl = fin.flags + sg[s].first;
-        E.ensure_filled(fl);
-        E.dev("compact_row_ids", [fl, cnt, ids, count, scratch, sb](cudaStream_t st) {
-            return sdb_compact_row_ids(fl, cnt, ids, count, scratch, sb, (sdb_stream_t)st);
-        });
+        std::vector<const void *> src;
+        std::vector<void *> dst;
+        std::vector<int> wide;
         for (Column *c : cols) {
             const Segment &seg = c->segments[s];
             if (c->is_aggregate_result) {
-                uint64_t *d = R.alloc<uint64_t>(cnt);
-                const uint64_t *src = seg.agg;
-                E.dev("gather", [src, ids, count, d, cnt](cudaStream_t st) {
-                    return sdb_gather_u64(src, ids, count, d, cnt, (sdb_stream_t)st);
-                });
-                o.dev.push_back(d);
+                src.push_back(seg.agg);
+                dst.push_back(R.alloc<uint64_t>(cnt));
+                wide.push_back(1);
             } else {
-                int32_t *d = R.alloc<int32_t>(cnt);
-                const int32_t *src = seg.data;
-                E.dev("gather", [src, ids, count, d, cnt](cudaStream_t st) {
-                    return sdb_gather_i32(src, ids, count, d, cnt, (sdb_stream_t)st);
-                });
-                o.dev.push_back(d);
+                src.push_back(seg.data);
+                dst.push_back(R.alloc<int32_t>(cnt));
+                wide.push_back(0);
             }
         }
+        o.dev = dst;
         pr.segs.push_back(o);
+        // a group-by result: straight from its occupancy words
+        auto oc = E.from_occ.find(fl0);
+        const bool occ = oc != E.from_occ.end();
+        const void *flags = occ ? static_cast<const void *>(oc->second.first) : fl0;
+        if (!occ) E.ensure_filled(fl0);
+        if (cnt <= 65536 && cols.size() <= 8) {  // one launch
+            E.dev("compact_gather", [flags, occ, cnt, src, wide, dst, count](cudaStream_t st) {
+                return occ ? sdb_compact_gather_occ(static_cast<const uint32_t *>(flags), cnt, (int)src.size(), src.data(),
+                                                    wide.data(), dst.data(), count, (sdb_stream_t)st)
+                           : sdb_compact_gather(static_cast<const uint8_t *>(flags), cnt, (int)src.size(), src.data(),
+                                                wide.data(), dst.data(), count, (sdb_stream_t)st);
+            });
+            continue;
+        }
+        void *scratch = E.mm.alloc<uint8_t>(sdb_compact_scratch_bytes(cnt));
+        E.dev("compact_gather", [flags, occ, cnt, src, wide, dst, count, scratch](cudaStream_t st) {
+            return sdb_compact_gather_large(flags, occ, cnt, (int)src.size(), src.data(), wide.data(), dst.data(), count,
+                                            scratch, st);
+        });
     }
     return pr;
 }

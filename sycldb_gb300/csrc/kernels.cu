@@ -658,35 +658,60 @@ struct ProbeFullOA {
 };
 
 // ---------------------------------------------------------------- K14, K15
+// Ordered compaction: the flagged rows of a segment, in row order, as row ids
+// and / or gathered columns.  Two launches: the tiles' counts, then every tile
+// adds up the counts of the tiles before it (at most 4096 words, from L2) and
+// writes its rows.  Streams the flags twice; the second time they come from
+// L2 up to its size.  The row list in shared memory makes the gathers and the
+// stores consecutive.  30 M flags, 0.36 % set, two int32 columns: 32 us; with a
+// one-block scan of the counts between the two and a gather launch per
+// column on top it was 65.
 constexpr int kCompactRowsPerThread = 16;
-constexpr int kCompactChunk = kThreads * kCompactRowsPerThread;  // rows per block-chunk
+constexpr int kCompactChunk = kThreads * kCompactRowsPerThread;  // rows per count that callers' scratch is sized for
+constexpr uint32_t kCompactRows = 4 * kCompactChunk;              // rows a block lists at a time
+constexpr uint32_t kCompactTiles = 4096;                          // most tiles of a launch
+constexpr int kCompactCols = 8;                                   // columns gathered by one launch
 
-__device__ __forceinline__ uint32_t count16(const uint8_t *flags, uint64_t r0, uint64_t n)
-{
-    if (r0 + 16 <= n) {
-        uint4 w = *reinterpret_cast<const uint4 *>(flags + r0);
-        return __popc(nz_bits4(w.x)) + __popc(nz_bits4(w.y)) + __popc(nz_bits4(w.z)) + __popc(nz_bits4(w.w));
-    }
-    uint32_t c = 0;
-    for (uint64_t r = r0; r < n; r++) c += flags[r] != 0;
-    return c;
-}
+struct Compact {
+    const void *flags;  // uint8 flags, or uint32 occupancy words (flag = word != 0)
+    uint64_t n;
+    uint32_t subs;      // a tile is `subs` times kCompactRows rows
+    uint32_t *counts;   // per tile
+    int32_t *ids;       // NULL: not wanted
+    uint32_t *count;
+    int32_t ncols;
+    const void *src[kCompactCols];
+    void *dst[kCompactCols];
+    int32_t wide[kCompactCols];  // 1: uint64 column
+};
 
-__device__ __forceinline__ uint32_t mask16(const uint8_t *flags, uint64_t r0, uint64_t n)
+// Flags of rows r0 .. r0 + 15 as a mask (r0 a multiple of 16, flags 16-byte aligned).
+template <typename F>
+__device__ __forceinline__ uint32_t mask16(const F *flags, uint64_t r0, uint64_t n)
 {
-    if (r0 + 16 <= n) {
-        uint4 w = *reinterpret_cast<const uint4 *>(flags + r0);
-        return nz_bits4(w.x) | (nz_bits4(w.y) << 4) | (nz_bits4(w.z) << 8) | (nz_bits4(w.w) << 12);
-    }
     uint32_t m = 0;
+    if (r0 + 16 <= n) {
+        const uint4 *q = reinterpret_cast<const uint4 *>(flags + r0);
+        if (sizeof(F) == 1) {
+            const uint4 w = q[0];
+            return nz_bits4(w.x) | (nz_bits4(w.y) << 4) | (nz_bits4(w.z) << 8) | (nz_bits4(w.w) << 12);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint4 w = q[j];
+            m |= ((w.x != 0) | ((w.y != 0) << 1) | ((w.z != 0) << 2) | ((w.w != 0) << 3)) << (4 * j);
+        }
+        return m;
+    }
     for (uint64_t r = r0; r < n; r++) m |= (uint32_t)(flags[r] != 0) << (r - r0);
     return m;
 }
 
 // Exclusive block scan of one value per thread; returns the block total in *total.
+template <int THREADS>
 __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *total)
 {
-    __shared__ uint32_t warp_tot[kThreads / 32];
+    __shared__ uint32_t warp_tot[THREADS / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     uint32_t x = v;
 #pragma unroll
@@ -696,67 +721,118 @@ __device__ __forceinline__ uint32_t block_exclusive_scan(uint32_t v, uint32_t *t
     }
     if (lane == 31) warp_tot[wid] = x;
     __syncthreads();
-    if (wid == 0) {
-        uint32_t t = lane < kThreads / 32 ? warp_tot[lane] : 0;
+    uint32_t base = 0, all = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, t, o);
-            if (lane >= o) t += y;
-        }
-        if (lane < kThreads / 32) warp_tot[lane] = t;  // inclusive prefix of warps
+    for (int w = 0; w < THREADS / 32; w++) {
+        const uint32_t t = warp_tot[w];
+        base += w < wid ? t : 0;
+        all += t;
     }
-    __syncthreads();
-    uint32_t base = wid ? warp_tot[wid - 1] : 0;
-    *total = warp_tot[kThreads / 32 - 1];
+    *total = all;
     __syncthreads();
     return base + x - v;
 }
 
-__global__ void __launch_bounds__(kThreads) k_compact_count(const uint8_t *flags, uint64_t n, uint32_t *block_counts,
-                                                            uint64_t nchunks)
+// Writes the rows list[0 .. total) (offsets from r0) at positions pos ..
+template <int THREADS>
+__device__ __forceinline__ void put_rows(const Compact &a, const uint16_t *list, uint32_t total, uint64_t r0, uint32_t pos)
 {
-    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const uint64_t r0 = c * kCompactChunk + (uint64_t)threadIdx.x * kCompactRowsPerThread;
-        uint32_t v = r0 < n ? count16(flags, r0, n) : 0;
-        uint32_t tot;
-        block_exclusive_scan(v, &tot);
-        if (threadIdx.x == 0) block_counts[c] = tot;
+    for (uint32_t i = threadIdx.x; i < total; i += THREADS) {
+        const uint64_t r = r0 + list[i];
+        const uint32_t at = pos + i;
+        if (a.ids) a.ids[at] = (int32_t)r;
+        // every column loaded before any store
+        uint64_t v[kCompactCols];
+#pragma unroll
+        for (int c = 0; c < kCompactCols; c++)
+            if (c < a.ncols)
+                v[c] = a.wide[c] ? static_cast<const uint64_t *>(a.src[c])[r]
+                                 : (uint64_t)(uint32_t)static_cast<const int32_t *>(a.src[c])[r];
+#pragma unroll
+        for (int c = 0; c < kCompactCols; c++)
+            if (c < a.ncols) {
+                if (a.wide[c]) static_cast<uint64_t *>(a.dst[c])[at] = v[c];
+                else static_cast<int32_t *>(a.dst[c])[at] = (int32_t)(uint32_t)v[c];
+            }
     }
 }
 
-// Single block: exclusive scan of the chunk counts in place; *count = total.
-__global__ void __launch_bounds__(kThreads) k_compact_scan(uint32_t *block_counts, uint64_t nchunks, uint32_t *count)
+template <typename F>
+__global__ void __launch_bounds__(kThreads) k_compact_count(const __grid_constant__ Compact a)
 {
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0;
-    __syncthreads();
-    for (uint64_t base = 0; base < nchunks; base += kThreads) {
-        const uint64_t i = base + threadIdx.x;
-        uint32_t v = i < nchunks ? block_counts[i] : 0;
-        uint32_t tot;
-        uint32_t ex = block_exclusive_scan(v, &tot);
-        if (i < nchunks) block_counts[i] = carry + ex;
-        __syncthreads();
-        if (threadIdx.x == 0) carry += tot;
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *count = carry;
-}
-
-__global__ void __launch_bounds__(kThreads) k_compact_write(const uint8_t *flags, uint64_t n, const uint32_t *offsets,
-                                                            uint64_t nchunks, int32_t *ids)
-{
-    for (uint64_t c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const uint64_t r0 = c * kCompactChunk + (uint64_t)threadIdx.x * kCompactRowsPerThread;
-        uint32_t m = r0 < n ? mask16(flags, r0, n) : 0;
-        uint32_t tot;
-        uint32_t pos = offsets[c] + block_exclusive_scan(__popc(m), &tot);
-        while (m) {
-            int j = __ffs(m) - 1;
-            ids[pos++] = (int32_t)(r0 + j);
-            m &= m - 1;
+    const uint64_t t0 = (uint64_t)blockIdx.x * a.subs * kCompactRows;
+    uint32_t c = 0;
+    for (uint32_t s = 0; s < a.subs; s++) {
+        const uint64_t r0 = t0 + (uint64_t)s * kCompactRows + threadIdx.x * 16u;
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint64_t r = r0 + (uint64_t)j * kCompactChunk;
+            if (r < a.n) c += __popc(mask16(static_cast<const F *>(a.flags), r, a.n));
         }
     }
+    uint32_t total;
+    block_exclusive_scan<kThreads>(c, &total);
+    if (threadIdx.x == 0) a.counts[blockIdx.x] = total;
+}
+
+template <typename F>
+__global__ void __launch_bounds__(kThreads) k_compact_write(const __grid_constant__ Compact a)
+{
+    __shared__ uint16_t s_list[kCompactRows];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t t0 = (uint64_t)blockIdx.x * a.subs * kCompactRows;
+    // warp w lists rows [2048 w, 2048 w + 2048): four steps of 16 rows per lane
+    uint32_t m[4];
+    auto load = [&](uint64_t r0) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const uint64_t r = r0 + warp * 2048u + j * 512u + lane * 16u;
+            m[j] = r < a.n ? mask16(static_cast<const F *>(a.flags), r, a.n) : 0;
+        }
+    };
+    load(t0);  // in flight with the counts
+    uint32_t before = 0, pos;
+#pragma unroll 4
+    for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kThreads) before += a.counts[t];
+    block_exclusive_scan<kThreads>(before, &pos);
+    for (uint32_t s = 0; s < a.subs; s++) {
+        const uint64_t r0 = t0 + (uint64_t)s * kCompactRows;
+        if (r0 >= a.n) break;  // block-uniform
+        if (s) load(r0);
+        // the steps' lane prefixes, two 16-bit counts a word (at most 512 each)
+        uint32_t x = __popc(m[0]) | (__popc(m[1]) << 16), y = __popc(m[2]) | (__popc(m[3]) << 16);
+        const uint32_t cx = x, cy = y;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t px = __shfl_up_sync(0xffffffffu, x, o), py = __shfl_up_sync(0xffffffffu, y, o);
+            if (lane >= (uint32_t)o) {
+                x += px;
+                y += py;
+            }
+        }
+        const uint32_t tx = __shfl_sync(0xffffffffu, x, 31), ty = __shfl_sync(0xffffffffu, y, 31);
+        const uint32_t sums[4] = {tx & 0xffffu, tx >> 16, ty & 0xffffu, ty >> 16};
+        x -= cx;
+        y -= cy;
+        const uint32_t lanes[4] = {x & 0xffffu, x >> 16, y & 0xffffu, y >> 16};
+        uint32_t total;
+        uint32_t at = block_exclusive_scan<kThreads>(lane == 0 ? sums[0] + sums[1] + sums[2] + sums[3] : 0, &total);
+        at = __shfl_sync(0xffffffffu, at, 0);  // lane 0's prefix is its warp's
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            uint32_t q = at + lanes[j], f = m[j];
+            while (f) {
+                s_list[q++] = (uint16_t)(warp * 2048u + j * 512u + lane * 16u + (uint32_t)__ffs(f) - 1u);
+                f &= f - 1;
+            }
+            at += sums[j];
+        }
+        __syncthreads();
+        put_rows<kThreads>(a, s_list, total, r0, pos);
+        pos += total;
+        __syncthreads();  // the list has been read
+    }
+    if (blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) *a.count = pos;
 }
 
 template <typename T>
@@ -768,96 +844,45 @@ __global__ void __launch_bounds__(kMaxBlock) k_gather(const T *src, const int32_
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < c; i += stride) dst[i] = src[ids[i]];
 }
 
-// Ordered compaction and the gathers of every result column of a small
-// segment (a group-by result) in one block of 1024 threads: thread t owns
-// rows [t*per, (t+1)*per), counts its flagged rows, a block scan gives its
-// first output position, then it copies its rows' values in row order.
+// The same for a small segment (a group-by result) in one launch: every block
+// counts the flags before its 2048 rows itself.  4375 slots, four columns:
+// 6.3 us, 8.5 in one block of 1024 threads with a thread's rows side by side.
 constexpr uint32_t kSmallCompactMax = 65536;
-static_assert(kSmallCompactMax <= 1024u * 64u, "k_compact_gather_small keeps a thread's flags in a 64-bit mask");
-constexpr int kSmallCompactCols = 8;
-struct SmallCompact {
-    const void *flags;  // uint8 flags, or uint32 occupancy words (flag = word != 0)
-    uint32_t n;
-    int32_t ncols;
-    const void *src[kSmallCompactCols];
-    void *dst[kSmallCompactCols];
-    int32_t wide[kSmallCompactCols];  // 1: uint64 column
-    uint32_t *count;
-};
+constexpr int kSmallCompactThreads = 512;
 
-template <typename F>
-__global__ void __launch_bounds__(1024) k_compact_gather_small(const __grid_constant__ SmallCompact a)
+template <typename F, bool VEC>
+__global__ void __launch_bounds__(kSmallCompactThreads) k_compact_gather_small(const __grid_constant__ Compact a)
 {
+    __shared__ uint16_t s_list[4 * kSmallCompactThreads];
     const F *flags = static_cast<const F *>(a.flags);
-    __shared__ uint32_t s_warp[32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t per = (a.n + 1023u) / 1024u;  // at most 64: n <= kSmallCompactMax
-    const uint32_t b = min(threadIdx.x * per, a.n), e = min(b + per, a.n);
-    // the thread's run of flags as a bit mask, eight independent loads at a
-    // time (one latency per eight flags instead of one per flag)
-    uint64_t m = 0;
-    for (uint32_t j = b; j < e; j += 8) {
-        F f[8];
-#pragma unroll
-        for (int k = 0; k < 8; k++) f[k] = j + k < e ? flags[j + k] : F(0);
-#pragma unroll
-        for (int k = 0; k < 8; k++) m |= (uint64_t)(f[k] != 0) << (j - b + k);
-    }
-    const uint32_t cnt = __popcll(m);
-    uint32_t x = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= (uint32_t)o) x += y;
-    }
-    if (lane == 31) s_warp[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t w = s_warp[lane];
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= (uint32_t)o) w += y;
+    const uint32_t n = (uint32_t)a.n, r0 = blockIdx.x * 4u * kSmallCompactThreads;
+    // flags of rows r .. r + 3 as a mask
+    auto mask4 = [&](uint32_t r) -> uint32_t {
+        if (VEC && r + 4 <= n) {
+            if (sizeof(F) == 1) return nz_bits4(*reinterpret_cast<const uint32_t *>(flags + r));
+            const uint4 w = *reinterpret_cast<const uint4 *>(flags + r);
+            return (w.x != 0) | ((w.y != 0) << 1) | ((w.z != 0) << 2) | ((w.w != 0) << 3);
         }
-        s_warp[lane] = w;
-    }
-    __syncthreads();
-    uint32_t pos = x - cnt + (warp ? s_warp[warp - 1] : 0);
-    if (threadIdx.x == 1023) *a.count = pos + cnt;
-    // two live rows per round, every column of both loaded before any store
+        uint32_t m = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < 4; j++)
+            if (r + j < n) m |= (uint32_t)(flags[r + j] != 0) << j;
+        return m;
+    };
+    uint32_t before = 0;
+    uint32_t m = mask4(r0 + threadIdx.x * 4u);
+#pragma unroll 8
+    for (uint32_t b = 0; b < blockIdx.x; b++) before += __popc(mask4((b * kSmallCompactThreads + threadIdx.x) * 4u));
+    uint32_t pos, total;
+    block_exclusive_scan<kSmallCompactThreads>(before, &pos);
+    uint32_t at = block_exclusive_scan<kSmallCompactThreads>(__popc(m), &total);
     while (m) {
-        const uint32_t i0 = b + (uint32_t)__ffsll((long long)m) - 1u;
+        s_list[at++] = (uint16_t)(threadIdx.x * 4u + (uint32_t)__ffs(m) - 1u);
         m &= m - 1;
-        const bool two = m != 0;
-        const uint32_t i1 = two ? b + (uint32_t)__ffsll((long long)m) - 1u : i0;
-        if (two) m &= m - 1;
-        uint64_t v0[kSmallCompactCols], v1[kSmallCompactCols];
-#pragma unroll
-        for (int c = 0; c < kSmallCompactCols; c++) {
-            if (c < a.ncols) {
-                if (a.wide[c]) {
-                    v0[c] = static_cast<const uint64_t *>(a.src[c])[i0];
-                    v1[c] = static_cast<const uint64_t *>(a.src[c])[i1];
-                } else {
-                    v0[c] = (uint32_t) static_cast<const int32_t *>(a.src[c])[i0];
-                    v1[c] = (uint32_t) static_cast<const int32_t *>(a.src[c])[i1];
-                }
-            }
-        }
-#pragma unroll
-        for (int c = 0; c < kSmallCompactCols; c++) {
-            if (c < a.ncols) {
-                if (a.wide[c]) {
-                    static_cast<uint64_t *>(a.dst[c])[pos] = v0[c];
-                    if (two) static_cast<uint64_t *>(a.dst[c])[pos + 1] = v1[c];
-                } else {
-                    static_cast<int32_t *>(a.dst[c])[pos] = (int32_t)(uint32_t)v0[c];
-                    if (two) static_cast<int32_t *>(a.dst[c])[pos + 1] = (int32_t)(uint32_t)v1[c];
-                }
-            }
-        }
-        pos += two ? 2u : 1u;
     }
+    __syncthreads();
+    put_rows<kSmallCompactThreads>(a, s_list, total, r0, pos);
+    if (blockIdx.x + 1 == gridDim.x && threadIdx.x == 0) *a.count = pos + total;
 }
 
 // ---------------------------------------------------------------- data gen
@@ -911,6 +936,24 @@ bool nat8(const void *p) { return sdb::aligned(p, 8); }
 }  // namespace
 
 // ============================================================== C ABI
+namespace {
+// The compaction's launches (count_first: the tiles' counts too, else they are
+// there from an earlier call over the same flags).
+void launch_compact(Compact &a, bool occ, bool count_first, cudaStream_t s)
+{
+    const uint64_t lists = (a.n + kCompactRows - 1) / kCompactRows;
+    a.subs = (uint32_t)((lists + kCompactTiles - 1) / kCompactTiles);
+    const unsigned tiles = (unsigned)((lists + a.subs - 1) / a.subs);
+    if (occ) {
+        if (count_first) k_compact_count<uint32_t><<<tiles, kThreads, 0, s>>>(a);
+        k_compact_write<uint32_t><<<tiles, kThreads, 0, s>>>(a);
+    } else {
+        if (count_first) k_compact_count<uint8_t><<<tiles, kThreads, 0, s>>>(a);
+        k_compact_write<uint8_t><<<tiles, kThreads, 0, s>>>(a);
+    }
+}
+}  // namespace
+
 extern "C" {
 
 int sdb_fill_u8(uint8_t *flags, uint64_t n, uint8_t v, sdb_stream_t stream)
@@ -1217,15 +1260,16 @@ int sdb_compact_row_ids(const uint8_t *flags, uint64_t n, int32_t *ids, uint32_t
     }
     if (!flags || !ids) return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_row_ids: NULL buffer");
     if (!sdb::aligned(flags, 16)) return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_row_ids: flags must be 16-byte aligned");
-    const uint64_t nchunks = (n + kCompactChunk - 1) / kCompactChunk;
     if (!scratch || scratch_bytes < sdb_compact_scratch_bytes(n))
         return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_row_ids: scratch needs %zu bytes", sdb_compact_scratch_bytes(n));
-    uint32_t *bc = static_cast<uint32_t *>(scratch);
-    const unsigned grid = (unsigned)std::min<uint64_t>(nchunks, (uint64_t)sdb::device_sms() * 8);
-    k_compact_count<<<grid, kThreads, 0, s>>>(flags, n, bc, nchunks);
-    k_compact_scan<<<1, kThreads, 0, s>>>(bc, nchunks, count);
-    k_compact_write<<<grid, kThreads, 0, s>>>(flags, n, bc, nchunks, ids);
-    sdb_count_launches(2);
+    Compact a{};
+    a.flags = flags;
+    a.n = n;
+    a.counts = static_cast<uint32_t *>(scratch);
+    a.ids = ids;
+    a.count = count;
+    launch_compact(a, false, true, s);
+    sdb_count_launches(1);
     return sdb_check_launch("sdb_compact_row_ids");
 }
 
@@ -1293,14 +1337,14 @@ static int compact_gather(const void *flags, bool occ, uint64_t n, int ncols, co
 {
     if (n > kSmallCompactMax) return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather: n=%llu exceeds %u",
                                                    (unsigned long long)n, kSmallCompactMax);
-    if (ncols < 0 || ncols > kSmallCompactCols || (ncols && (!src || !wide || !dst)))
-        return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather: 0..%d columns", kSmallCompactCols);
+    if (ncols < 0 || ncols > kCompactCols || (ncols && (!src || !wide || !dst)))
+        return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather: 0..%d columns", kCompactCols);
     if (!count || (n && !flags)) return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather: NULL flags or count");
     if (occ && !sdb::aligned(flags, 4)) return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather_occ: occ misaligned");
     if (!sdb::aligned(count, 4)) return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather: count misaligned");
-    SmallCompact a;
+    Compact a{};
     a.flags = flags;
-    a.n = (uint32_t)n;
+    a.n = n;
     a.ncols = ncols;
     a.count = count;
     for (int c = 0; c < ncols; c++) {
@@ -1311,10 +1355,11 @@ static int compact_gather(const void *flags, bool occ, uint64_t n, int ncols, co
         a.dst[c] = dst[c];
         a.wide[c] = wide[c] ? 1 : 0;
     }
-    if (occ)
-        k_compact_gather_small<uint32_t><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
-    else
-        k_compact_gather_small<uint8_t><<<1, 1024, 0, (cudaStream_t)stream>>>(a);
+    const unsigned blocks = (unsigned)std::max<uint64_t>(1, (n + 4 * kSmallCompactThreads - 1) / (4 * kSmallCompactThreads));
+    const bool vec = sdb::aligned(flags, occ ? 16 : 4);
+    auto kern = occ ? (vec ? k_compact_gather_small<uint32_t, true> : k_compact_gather_small<uint32_t, false>)
+                    : (vec ? k_compact_gather_small<uint8_t, true> : k_compact_gather_small<uint8_t, false>);
+    kern<<<blocks, kSmallCompactThreads, 0, (cudaStream_t)stream>>>(a);
     return sdb_check_launch("sdb_compact_gather");
 }
 
@@ -1438,3 +1483,31 @@ int sdb_op_tune_get(int op_kernel, uint64_t rows, int *block, int *blocks_per_sm
 }
 
 }  // extern "C"
+
+// The flagged rows of a segment of any size (flags or occupancy words, 16-byte
+// aligned) gathered from any number of columns: what sdb_compact_row_ids and
+// one sdb_gather_* per column give together.  Scratch as for
+// sdb_compact_row_ids.  For the executor's results above sdb_compact_gather's
+// limits.
+int sdb_compact_gather_large(const void *flags, bool occ, uint64_t n, int ncols, const void *const *src, const int *wide,
+                             void *const *dst, uint32_t *count, void *scratch, cudaStream_t s)
+{
+    Compact a{};
+    a.flags = flags;
+    a.n = n;
+    a.counts = static_cast<uint32_t *>(scratch);
+    a.count = count;
+    int launches = 0;
+    for (int c0 = 0; c0 == 0 || c0 < ncols; c0 += kCompactCols) {
+        a.ncols = std::min(kCompactCols, ncols - c0);
+        for (int c = 0; c < a.ncols; c++) {
+            a.src[c] = src[c0 + c];
+            a.dst[c] = dst[c0 + c];
+            a.wide[c] = wide[c0 + c];
+        }
+        launch_compact(a, occ, c0 == 0, s);
+        launches += c0 == 0 ? 2 : 1;
+    }
+    sdb_count_launches((unsigned)launches - 1);
+    return sdb_check_launch("sdb_compact_gather_large");
+}
