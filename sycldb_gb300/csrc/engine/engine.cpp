@@ -52,6 +52,9 @@
 int sdb_set_error(int status, const char *fmt, ...);
 int sdb_compact_gather_large(const void *flags, bool occ, uint64_t n, int ncols, const void *const *src, const int *wide,
                              void *const *dst, uint32_t *count, void *scratch, cudaStream_t s);  // kernels.cu
+int sdb_sort_gather_small(const void *const *keys, const int *key_types, const int *descending, int nkeys,
+                          const uint32_t *count, uint64_t cap, int ncols, const void *const *src, const int *wide,
+                          void *const *dst, uint32_t *count_out, cudaStream_t s);  // sort.cu
 
 namespace sdb {
 
@@ -148,6 +151,13 @@ int32_t stoi_ref(const std::string &s)
         throw Error(SDB_ERR_INVALID, "SEARCH bound is not an integer: '" + s + "'");
     }
 }
+
+// Pinned bytes an engine keeps for its results: 65536 slots of a three-key
+// group-by (5 columns, 24 bytes a slot) and more; a result above it is copied.
+constexpr uint64_t kPinnedResult = 4u << 20;
+// Rows up to which an ordered result is sorted by counting (sdb_sort_rows's
+// small case), in the launch that gathers it.
+constexpr uint64_t kSmallOrdered = 4096;
 
 // ------------------------------------------------------------------ memory
 // Device bump allocator with a zeroed region of budget/64
@@ -259,6 +269,7 @@ public:
 
     // memory_manager::reset (operations/memory_manager.cpp:71-90): rewind and
     // re-zero what the zeroed region handed out.
+    void rewind() { used_ = 0; }
     void reset(cudaStream_t s)
     {
         used_ = 0;
@@ -824,6 +835,11 @@ struct Engine {
     }
     uint64_t seg = kDefaultSegment;
     MemoryManager mm;
+    // Pinned host memory for the results of plain executions: counts, and the
+    // columns of results of up to kPinnedResult bytes, written there by the
+    // compaction itself (one wait, no copy), other results' counts alone.
+    char *pinned = nullptr;
+    MemoryManager pin;
     std::map<std::string, std::unique_ptr<Table>> tables;
     // Tables being loaded from column files in the background: installed by
     // the first plan that scans them (activate).
@@ -1655,6 +1671,11 @@ struct PendingResult {
     std::vector<int> types;  // 0 int32, 1 uint64
     std::vector<PendingSeg> segs;
     std::vector<std::pair<int, int>> order;  // ORDER BY: (result column, descending), first key first
+    bool on_host = false;                    // plain execution: counts and columns are in the engine's pinned memory
+    // plain execution, ORDER BY of a small result: its count and ordered
+    // columns in pinned memory, there when the count is at most kSmallOrdered
+    bool sorted = false;
+    PendingSeg ordered;
 };
 
 }  // namespace sdb
@@ -2033,11 +2054,25 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
         break;
     }
     auto sg = fin.segs();
+    auto room = [&](uint64_t rows) {  // bytes of a segment's count and columns
+        uint64_t b = 256;
+        for (int t : pr.types) b += (rows * (t == 1 ? 8 : 4) + 511) & ~(uint64_t)255;
+        return b;
+    };
+    const bool order = !E.rmm && E.cfg.order_by && !pr.order.empty();
+    if (!E.rmm) {
+        // pinned memory when the whole capacity fits; a result to be ordered
+        // stays on the device for the sort
+        uint64_t all = 0;
+        for (auto &x : sg) all += room(x.second);
+        E.pin.rewind();
+        pr.on_host = !order && all <= E.pin.size();
+    }
+    MemoryManager &R = E.rmm ? *E.rmm : (pr.on_host ? E.pin : E.mm);
     for (size_t s = 0; s < sg.size(); s++) {
         const uint64_t cnt = sg[s].second;
         PendingSeg o;
         o.cap = cnt;
-        MemoryManager &R = E.rmm ? *E.rmm : E.mm;
         const uint8_t *fl0 = fin.flags + sg[s].first;
         uint32_t *count = R.alloc<uint32_t>(1);
         o.count = count;
@@ -2076,6 +2111,30 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
         E.dev("compact_gather", [flags, occ, cnt, src, wide, dst, count, scratch](cudaStream_t st) {
             return sdb_compact_gather_large(flags, occ, cnt, (int)src.size(), src.data(), wide.data(), dst.data(), count,
                                             scratch, st);
+        });
+    }
+    // A small ordered result (one segment): sorted and gathered into pinned
+    // memory by a launch that reads the count on the device, so that the host
+    // waits once; a larger one, known by its count, goes through sort_result.
+    if (order && pr.segs.size() == 1 && pr.types.size() <= 8 && pr.order.size() <= 16 &&
+        room(kSmallOrdered) <= E.pin.size()) {
+        const PendingSeg &o = pr.segs[0];
+        const uint64_t cap = std::min(o.cap, kSmallOrdered);
+        pr.ordered.cap = cap;
+        pr.ordered.count = E.pin.alloc<uint32_t>(1);
+        for (int t : pr.types) pr.ordered.dev.push_back(t == 1 ? (void *)E.pin.alloc<uint64_t>(cap) : (void *)E.pin.alloc<int32_t>(cap));
+        pr.sorted = true;
+        std::vector<const void *> keys;
+        std::vector<int> types, desc;
+        for (auto &k : pr.order) {
+            keys.push_back(o.dev[k.first]);
+            types.push_back(pr.types[k.first]);
+            desc.push_back(k.second);
+        }
+        E.dev("sort_rows", [&](cudaStream_t st) {
+            return sdb_sort_gather_small(keys.data(), types.data(), desc.data(), (int)keys.size(), o.count, cap,
+                                         (int)pr.types.size(), o.dev.data(), pr.types.data(), pr.ordered.dev.data(),
+                                         pr.ordered.count, st);
         });
     }
     return pr;
@@ -2154,9 +2213,21 @@ std::unique_ptr<sdb_result> execute_plan(Engine &E, const std::string &plan_text
     res->i32.resize(ncols);
     res->u64.resize(ncols);
     std::vector<uint32_t> counts(pr.segs.size());
-    for (size_t s = 0; s < pr.segs.size(); s++)
-        SDB_CUDA(cudaMemcpyAsync(&counts[s], pr.segs[s].count, sizeof(uint32_t), cudaMemcpyDeviceToHost, E.stream));
-    SDB_CUDA(cudaStreamSynchronize(E.stream));
+    uint32_t *host_counts = nullptr;  // for counts that are on the device: pinned, unless there are too many segments
+    if (!pr.on_host) {
+        if (pr.sorted) host_counts = pr.ordered.count;
+        else host_counts = counts.size() * sizeof(uint32_t) <= E.pin.size() ? E.pin.alloc<uint32_t>(counts.size()) : counts.data();
+        for (size_t s = 0; s < counts.size() && !pr.sorted; s++)
+            SDB_CUDA(cudaMemcpyAsync(host_counts + s, pr.segs[s].count, sizeof(uint32_t), cudaMemcpyDeviceToHost, E.stream));
+    }
+    SDB_CUDA(cudaEventRecord(E.plan_b, E.stream));
+    SDB_CUDA(cudaEventSynchronize(E.plan_b));
+    for (size_t s = 0; s < counts.size(); s++) counts[s] = pr.on_host ? *pr.segs[s].count : host_counts[s];
+    bool on_host = pr.on_host;
+    if (pr.sorted && counts[0] <= pr.ordered.cap) {
+        pr.segs.assign(1, pr.ordered);
+        on_host = true;
+    }
     uint64_t total = 0;
     for (auto c : counts) total += c;
     for (size_t ci = 0; ci < ncols; ci++) {
@@ -2165,22 +2236,25 @@ std::unique_ptr<sdb_result> execute_plan(Engine &E, const std::string &plan_text
         else
             res->i32[ci].resize(total);
     }
-    if (E.cfg.order_by && !pr.order.empty() && total > 1) sort_result(E, pr, counts, total);
+    if (!on_host && E.cfg.order_by && !pr.order.empty() && total > 1) sort_result(E, pr, counts, total);
     uint64_t base = 0;
     for (size_t s = 0; s < pr.segs.size(); s++) {
         for (size_t ci = 0; ci < ncols; ci++) {
             if (!counts[s]) continue;
-            if (res->types[ci] == 1)
-                SDB_CUDA(cudaMemcpyAsync(res->u64[ci].data() + base, pr.segs[s].dev[ci], counts[s] * sizeof(uint64_t),
-                                         cudaMemcpyDeviceToHost, E.stream));
+            const bool u64 = res->types[ci] == 1;
+            void *to = u64 ? (void *)(res->u64[ci].data() + base) : (void *)(res->i32[ci].data() + base);
+            const size_t bytes = counts[s] * (u64 ? sizeof(uint64_t) : sizeof(int32_t));
+            if (on_host)
+                std::memcpy(to, pr.segs[s].dev[ci], bytes);
             else
-                SDB_CUDA(cudaMemcpyAsync(res->i32[ci].data() + base, pr.segs[s].dev[ci], counts[s] * sizeof(int32_t),
-                                         cudaMemcpyDeviceToHost, E.stream));
+                SDB_CUDA(cudaMemcpyAsync(to, pr.segs[s].dev[ci], bytes, cudaMemcpyDeviceToHost, E.stream));
         }
         base += counts[s];
     }
-    SDB_CUDA(cudaEventRecord(E.plan_b, E.stream));
-    SDB_CUDA(cudaStreamSynchronize(E.stream));
+    if (!on_host) {
+        SDB_CUDA(cudaEventRecord(E.plan_b, E.stream));
+        SDB_CUDA(cudaEventSynchronize(E.plan_b));
+    }
     res->nrows = total;
     float ms = 0;
     SDB_CUDA(cudaEventElapsedTime(&ms, E.plan_a, E.plan_b));
@@ -2451,7 +2525,8 @@ void replay(sdb_batch &B, cudaStream_t main)
     mark(B.ev_c1);
     phase(&PlanRecord::post);
     // every plan's count and result columns, in one copy to the pinned mirror
-    if (B.rbytes) SDB_CUDA(cudaMemcpyAsync(B.host, B.rbase, B.rbytes, cudaMemcpyDeviceToHost, main));
+    // (unless they were written there)
+    if (B.rbytes && B.rbase != B.host) SDB_CUDA(cudaMemcpyAsync(B.host, B.rbase, B.rbytes, cudaMemcpyDeviceToHost, main));
 }
 
 // Where each plan's count and result columns sit in the result region (and
@@ -2520,7 +2595,12 @@ void batch_prepare(Engine &E, sdb_batch &B, const std::vector<std::string> &plan
 
     // real pass against an arena of exactly that size
     B.mm.init_sized(used + cb_bytes + 256, zused, E.stream);
-    B.rmm.init_sized(rused, 256, E.stream);
+    // the results' region is the pinned memory the host reads: the compactions
+    // write the rows there are, where a copy would move every column's
+    // capacity
+    B.host_bytes = std::max<size_t>(rused, 256);
+    SDB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&B.host), B.host_bytes, cudaHostAllocDefault));
+    B.rmm.init_external(B.host, B.host_bytes, B.host, 0);
     record_plans(E, B, B.mm, B.rmm, plans);
     pair_chains(E, B);
     if (!B.rec.chains.empty()) {
@@ -2533,8 +2613,6 @@ void batch_prepare(Engine &E, sdb_batch &B, const std::vector<std::string> &plan
     B.rbase = B.rmm.base();
     B.rbytes = B.rmm.used();
     layout_results(B, B.rbase);
-    B.host_bytes = std::max<size_t>(B.rbytes, 64);
-    SDB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&B.host), B.host_bytes, cudaHostAllocDefault));
 
     // streams and events; the plans' work is spread over up to 8 streams
     SDB_CUDA(cudaStreamCreateWithFlags(&B.bs, cudaStreamNonBlocking));
@@ -2809,6 +2887,8 @@ int sdb_engine_create(const sdb_engine_config *cfg, sdb_engine **out)
             budget = std::min<uint64_t>(std::max<uint64_t>(8ull << 30, tot / 2), (10ull << 30) + (512ull << 20));
         }
         E.mm.init(budget, E.stream);
+        SDB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&E.pinned), sdb::kPinnedResult, cudaHostAllocDefault));
+        E.pin.init_external(E.pinned, sdb::kPinnedResult, E.pinned, 0);
         E.prof.on = E.cfg.profile != 0;
         if (E.cfg.plan_cache < 0) throw sdb::Error(SDB_ERR_INVALID, "plan_cache must be >= 0");
         if (E.cfg.join_tables < 0 || E.cfg.join_tables > 2) throw sdb::Error(SDB_ERR_INVALID, "join_tables must be 0, 1 or 2");
@@ -2838,6 +2918,7 @@ int sdb_engine_destroy(sdb_engine *eng)
         for (auto p : t.second->owned) cudaFree(p);
     E.tables.clear();
     E.mm.release();
+    if (E.pinned) cudaFreeHost(E.pinned);
     if (E.plan_a) cudaEventDestroy(E.plan_a);
     if (E.plan_b) cudaEventDestroy(E.plan_b);
     if (E.aux) cudaStreamDestroy(E.aux);

@@ -9,6 +9,7 @@
 #include <memory>
 #include <stdexcept>
 #include <string>
+#include <string_view>
 #include <vector>
 
 namespace sdb {
@@ -29,14 +30,18 @@ struct Value {
     bool is_string() const { return kind == String; }
     bool is_number() const { return kind == Int || kind == Double; }
 
-    const Value *find(const std::string &key) const
+    const Value *find(std::string_view key) const
     {
         if (kind != Object) return nullptr;
         for (const auto &kv : obj)
             if (kv.first == key) return &kv.second;
         return nullptr;
     }
-    bool has(const std::string &key) const { return find(key) != nullptr && !find(key)->is_null(); }
+    bool has(std::string_view key) const
+    {
+        const Value *v = find(key);
+        return v && !v->is_null();
+    }
 
     int64_t as_int() const
     {
@@ -65,7 +70,8 @@ public:
 
     Value parse()
     {
-        Value v = value();
+        Value v;
+        value(v);
         ws();
         if (p_ != t_.size()) fail("trailing characters");
         return v;
@@ -104,20 +110,21 @@ private:
         return false;
     }
 
-    Value value()
+    // Reads the next value into `v` (a fresh one), in place.
+    void value(Value &v)
     {
         char c = peek();
-        Value v;
         if (c == '{') {
             p_++;
             v.kind = Value::Object;
-            if (peek() == '}') { p_++; return v; }
+            if (peek() == '}') { p_++; return; }
+            v.obj.reserve(4);
             for (;;) {
                 if (peek() != '"') fail("expected a key");
-                std::string k = str();
+                auto &kv = v.obj.emplace_back();
+                str(kv.first);
                 expect(':');
-                Value x = value();
-                v.obj.emplace_back(std::move(k), std::move(x));
+                value(kv.second);
                 char d = peek();
                 p_++;
                 if (d == '}') break;
@@ -126,9 +133,10 @@ private:
         } else if (c == '[') {
             p_++;
             v.kind = Value::Array;
-            if (peek() == ']') { p_++; return v; }
+            if (peek() == ']') { p_++; return; }
+            v.arr.reserve(4);
             for (;;) {
-                v.arr.push_back(value());
+                value(v.arr.emplace_back());
                 char d = peek();
                 p_++;
                 if (d == ']') break;
@@ -136,7 +144,7 @@ private:
             }
         } else if (c == '"') {
             v.kind = Value::String;
-            v.s = str();
+            str(v.s);
         } else if (lit("true")) {
             v.kind = Value::Bool;
             v.b = true;
@@ -147,16 +155,17 @@ private:
         } else {
             number(v);
         }
-        return v;
     }
 
-    std::string str()
+    void str(std::string &out)
     {
         expect('"');
-        std::string out;
         while (p_ < t_.size() && t_[p_] != '"') {
-            char c = t_[p_++];
-            if (c == '\\') {
+            const size_t run = p_;
+            while (p_ < t_.size() && t_[p_] != '"' && t_[p_] != '\\') p_++;
+            out.append(t_, run, p_ - run);
+            if (p_ < t_.size() && t_[p_] == '\\') {
+                p_++;
                 if (p_ >= t_.size()) fail("bad escape");
                 char e = t_[p_++];
                 switch (e) {
@@ -179,13 +188,10 @@ private:
                 }
                 default: fail("bad escape");
                 }
-            } else {
-                out += c;
             }
         }
         if (p_ >= t_.size()) fail("unterminated string");
         p_++;
-        return out;
     }
 
     void number(Value &v)
@@ -200,13 +206,14 @@ private:
             break;
         }
         if (s == p_) fail("unexpected character");
-        std::string num = t_.substr(s, p_ - s);
+        // the text is NUL-terminated, and a number ends at the first character
+        // that is not one of a number's
         if (is_double) {
             v.kind = Value::Double;
-            v.d = std::strtod(num.c_str(), nullptr);
+            v.d = std::strtod(t_.substr(s, p_ - s).c_str(), nullptr);
         } else {
             v.kind = Value::Int;
-            v.i = std::strtoll(num.c_str(), nullptr, 10);
+            v.i = std::strtoll(t_.c_str() + s, nullptr, 10);
         }
     }
 };

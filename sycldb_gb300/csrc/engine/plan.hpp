@@ -116,7 +116,7 @@ inline int64_t int_of(const json::Value &v, const char *what)
 
 // A name given as a string or as an object {"name": ...} (RelJson's
 // operators and aggregate functions) or {"type": ...} (RelJson's types).
-inline std::string name_of(const json::Value &v, const char *key, const char *what)
+inline const std::string &name_of(const json::Value &v, const char *key, const char *what)
 {
     if (v.is_string()) return v.s;
     if (v.is_object())
@@ -221,10 +221,11 @@ inline PlanResult plan_from_json(const std::string &text)
     const json::Value *rels = root.find("rels");
     if (!rels || !rels->is_array()) throw std::invalid_argument("plan: missing \"rels\" array");
     PlanResult plan;
+    plan.rels.reserve(rels->arr.size());
     for (const auto &r : rels->arr) {
-        RelNode n;
+        RelNode &n = plan.rels.emplace_back();
         if (!r.is_object()) throw std::invalid_argument("plan: rel must be an object");
-        n.id = r.find("id") ? detail::int_of(*r.find("id"), "id") : (int64_t)plan.rels.size();
+        n.id = r.find("id") ? detail::int_of(*r.find("id"), "id") : (int64_t)plan.rels.size() - 1;
         if (!r.find("relOp")) throw std::invalid_argument("plan: rel without relOp");
         n.relOp = detail::rel_op_of(*r.find("relOp"));
         // "tables" in the IDL shape, "table" in RelJson (SycldbJsonConverter.java:50-52)
@@ -250,7 +251,7 @@ inline PlanResult plan_from_json(const std::string &text)
                 if (x.has("name")) a.name = x.find("name")->as_string();
                 if (x.has("type")) a.type = detail::name_of(*x.find("type"), "type", "agg type");
                 if (x.has("distinct")) a.distinct = x.find("distinct")->as_bool();
-                n.aggs.push_back(a);
+                n.aggs.push_back(std::move(a));
             }
         if (const json::Value *co = r.find("collation"))
             for (const auto &x : co->arr) {
@@ -260,7 +261,6 @@ inline PlanResult plan_from_json(const std::string &text)
                 if (x.has("nulls")) c.nulls = detail::enum_of(*x.find("nulls"), kNulls, 2, "nulls");
                 n.collation.push_back(c);
             }
-        plan.rels.push_back(std::move(n));
     }
     for (size_t i = 0; i < plan.rels.size(); i++)
         if (plan.rels[i].id != (int64_t)i) throw std::invalid_argument("plan: rel ids must be 0..n-1 in order");

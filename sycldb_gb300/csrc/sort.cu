@@ -77,9 +77,28 @@ constexpr uint32_t kSmallSort = 4096;
 constexpr int kSmallRows = 4;
 constexpr int kSmallThreads = 128;
 
+// Columns to write in the order found, in place of the row ids: those of a
+// result whose row count is still on the device.
+struct SmallGather {
+    const uint32_t *count;  // rows (NULL: no gather)
+    uint32_t cap;           // nothing is ordered when there are more
+    uint32_t *count_out;
+    int ncols;
+    const void *src[8];
+    void *dst[8];
+    uint8_t wide[8];
+};
+
+template <bool GATHER>
 __global__ void __launch_bounds__(kSmallThreads) k_sort_small(const __grid_constant__ SortKeys K, uint32_t n,
-                                                                uint32_t *__restrict__ perm)
+                                                                uint32_t *__restrict__ perm,
+                                                                const __grid_constant__ SmallGather G)
 {
+    if (GATHER) {
+        n = *G.count;
+        if (blockIdx.x == 0 && threadIdx.x == 0) *G.count_out = n;
+        if (n > G.cap) return;
+    }
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t r0 = (blockIdx.x * (kSmallThreads / 32) + (threadIdx.x >> 5)) * kSmallRows;
     if (r0 >= n) return;  // warp-uniform
@@ -112,7 +131,13 @@ __global__ void __launch_bounds__(kSmallThreads) k_sort_small(const __grid_const
 #pragma unroll
     for (int q = 0; q < kSmallRows; q++) {
         const uint32_t at = __reduce_add_sync(0xffffffffu, before[q]);
-        if (lane == 0 && r0 + q < n) perm[at] = r0 + q;
+        if (r0 + q >= n) break;
+        if (!GATHER) {
+            if (lane == 0) perm[at] = r0 + q;
+        } else if (lane < (uint32_t)G.ncols) {
+            if (G.wide[lane]) static_cast<uint64_t *>(G.dst[lane])[at] = static_cast<const uint64_t *>(G.src[lane])[r0 + q];
+            else static_cast<int32_t *>(G.dst[lane])[at] = static_cast<const int32_t *>(G.src[lane])[r0 + q];
+        }
     }
 }
 
@@ -766,7 +791,7 @@ int sdb_sort_rows(const void *const *keys, const int *key_types, const int *desc
     const uint32_t n32 = (uint32_t)n;
     if (n <= kSmallSort) {
         constexpr uint32_t per_block = kSmallThreads / 32 * kSmallRows;
-        k_sort_small<<<(n32 + per_block - 1) / per_block, kSmallThreads, 0, s>>>(K, n32, perm);
+        k_sort_small<false><<<(n32 + per_block - 1) / per_block, kSmallThreads, 0, s>>>(K, n32, perm, SmallGather{});
         return sdb_check_launch("sdb_sort_rows");
     }
     Scratch sc;
@@ -828,3 +853,37 @@ int sdb_sort_rows(const void *const *keys, const int *key_types, const int *desc
 }
 
 }  // extern "C"
+
+// The rows of a result (*count of them, on the device, at most cap to be
+// ordered; cap <= 4096, up to 8 columns) written to dst in the order of the
+// keys, *count_out = *count: sdb_sort_rows and a gather per column in one
+// launch that needs no count on the host.  With more than cap rows only the
+// count is written.
+int sdb_sort_gather_small(const void *const *keys, const int *key_types, const int *descending, int nkeys,
+                          const uint32_t *count, uint64_t cap, int ncols, const void *const *src, const int *wide,
+                          void *const *dst, uint32_t *count_out, cudaStream_t s)
+{
+    if (nkeys < 1 || nkeys > kMaxKeys || cap > kSmallSort || ncols < 0 || ncols > 8)
+        return sdb_set_error(SDB_ERR_INVALID, "sdb_sort_gather_small: limits exceeded");
+    SortKeys K{};
+    K.n = nkeys;
+    for (int k = 0; k < nkeys; k++) {
+        K.col[k] = keys[k];
+        K.wide[k] = key_types[k] ? 1 : 0;
+        K.desc[k] = descending[k] ? 1 : 0;
+    }
+    SmallGather G{};
+    G.count = count;
+    G.cap = (uint32_t)cap;
+    G.count_out = count_out;
+    G.ncols = ncols;
+    for (int c = 0; c < ncols; c++) {
+        G.src[c] = src[c];
+        G.dst[c] = dst[c];
+        G.wide[c] = wide[c] ? 1 : 0;
+    }
+    constexpr uint32_t per_block = kSmallThreads / 32 * kSmallRows;
+    const uint32_t blocks = std::max<uint32_t>(1, ((uint32_t)cap + per_block - 1) / per_block);
+    k_sort_small<true><<<blocks, kSmallThreads, 0, s>>>(K, 0, nullptr, G);
+    return sdb_check_launch("sdb_sort_rows");
+}

@@ -78,3 +78,31 @@ def test_results_above_the_one_launch_limits(mode, seg):
                 assert got.canonical() == want
             if mode == "ordered" and plan is rows:
                 assert np.all(np.diff(got.columns[1].astype(np.int64)) >= 0)
+
+
+@pytest.mark.parametrize("qty,seg", [(2, 0), (8, 0), (9, 0), (30, 0), (8, 1 << 17)])
+def test_ordered_results_around_the_counted_sort_limit(qty, seg):
+    """ORDER BY (descending price, then date) of a filter's rows: below, at
+    about and above 4096 of them, and of a group-by; the same rows as without."""
+    ds = datasets.dataset(0.05)
+    b = plans.PlanBuilder()
+    b.scan("lineorder")
+    b.filter(plans.AND(plans.expr("<", plans.col(8), plans.lit(qty)), plans.search(11, 4, 5)))
+    b.project([plans.col(5), plans.col(9)])
+    b.rels.append({"id": len(b.rels), "relOp": "SORT",
+                   "collation": [{"field": 1, "direction": "DESCENDING"}, {"field": 0, "direction": "ASCENDING"}]})
+    rows, star = b.plan(), plans.plan_star(1, 3)
+    with Engine(arena_bytes=1 << 30, segment_rows=seg, order_by=True) as eng, \
+            Engine(arena_bytes=1 << 30, segment_rows=seg) as plain:
+        for name, cols in ds.items():
+            eng.load_table(name, cols)
+            plain.load_table(name, cols)
+        for _ in range(2):
+            got, base = eng.execute(rows), plain.execute(rows)
+            date, price = base.columns
+            at = np.lexsort((date, -price.astype(np.int64)))  # stable: ties keep row order
+            assert np.array_equal(got.columns[0], date[at]) and np.array_equal(got.columns[1], price[at])
+            g, p = eng.execute(star), plain.execute(star)
+            at = np.lexsort((p.columns[1], p.columns[0]))
+            for x, y in zip(g.columns, p.columns):
+                assert np.array_equal(x, y[at])
