@@ -365,12 +365,14 @@ int sdb_fused_chain(const sdb_chain_desc *chain, sdb_stream_t stream);
  * the next tile, so the one-row-per-lane ops run on full warps (chains whose
  * later ops write no column).  7: as 6, and the rows that survive the first
  * op after the compaction are compacted again, across lanes in registers,
- * so the later ops and the terminal run on full warps.  8: as 7, and the
- * columns that only the ops after that second compaction read are not
- * staged: a surviving row carries its row number and loads them there
- * (only the sectors holding such rows are read; chains under 2^31 rows,
- * else as 7).  Shapes without a
- * specialised pass fall back to the general pass.  Default (and an unset
+ * so the later ops and the terminal run on full warps.  8: the
+ * chain's late form -- the tests of its first two ops (a probe that gives a
+ * value tests its table's hits) on eight rows per thread, the rows that are
+ * left queued by row number, and every column the later ops read loaded for
+ * those rows alone (only the sectors holding such rows; chains under 2^31
+ * rows, else as 7).  Shapes without a
+ * specialised pass fall back to the general pass, or (chains whose flags only
+ * shrink) to the sieve, the late form's run-time counterpart.  Default (and an unset
  * tuning entry): 5. */
 int sdb_fused_chain_variant(const sdb_chain_desc *chain, int variant, sdb_stream_t stream);
 /* Tuning table used by sdb_fused_chain: variant for chains with this

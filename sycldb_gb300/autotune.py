@@ -10,8 +10,9 @@ The fused chain has nine kernel variants (``sdb_fused_chain_variant``):
   6      as 5, surviving rows that do not fill a warp carried into the next tile
   7      as 6, and the rows that survive the first row-per-lane op compacted
          again (across lanes, in registers) so the later ops run on full warps
-  8      as 7, and the columns that only the ops after that second compaction
-         read are not staged: each surviving row loads them by row number
+  8      the chain's late form: its first two ops tested on 8 rows per thread,
+         the rows that are left queued by row number, every column the later ops
+         read loaded for those rows alone
 
 The fused passes keep 256 threads per block: their copy ring, per-warp row
 lists and tile shape (256 x 4 rows) are laid out for it, and the variants

@@ -778,17 +778,14 @@ namespace dense {
 // lo <= a <= hi (empty when lo > hi).
 __device__ __forceinline__ bool in_range(int32_t a, int32_t lo, int32_t hi) { return a >= lo && a <= hi; }
 
-constexpr int kItems = 4;  // rows per thread per tile of the passes without late slots
-// Rows per thread per tile: CARRY 3 (late slots, two staged columns) takes 8
-// -- the same shared memory per stage as four columns of 4 rows -- the others
-// 4.  A thread copies items / 4 16-byte pieces per staged column and tile.
-template <int CARRY>
-__host__ __device__ constexpr int items_of() { return CARRY == 3 ? 8 : kItems; }
+// An op kind of the late passes, beside the SDB_OP_* ones: a full probe that
+// only tests the row; its value is read later, by the same probe on the rows
+// that are left.
+constexpr int K_HIT = 7;
+
+constexpr int kItems = 4;  // rows per thread per tile
+constexpr int kQ = kItems / 4;  // 16-byte pieces a thread copies per column and tile
 constexpr int kSlots = 4;
-// Slots per ring stage: CARRY 3 stages only its first two slots (the late
-// ones, renumbered last, are not staged) and spends the space on more stages.
-template <int CARRY>
-__host__ __device__ constexpr int stage_slots() { return CARRY == 3 ? 2 : kSlots; }
 constexpr int kMaxOps = 8;
 
 struct Src {
@@ -817,10 +814,10 @@ struct Launch {
     Src value;
     uint64_t *sum_out;
     int32_t n_keys;
-    uint32_t tail_slots;  // slots read after the first op (bit s = slot s): what a carried row keeps
-    uint32_t late_slots;  // CARRY 3: tail slots read only after the second compaction level -- not
-                          // staged; a row carries its row number there and the second level loads them
-    int32_t nstaged;      // slots staged by the copy ring: 0 .. nstaged-1 (all nslot but for CARRY 3)
+    uint32_t tail_slots;  // slots read after the dense ops (bit s = slot s): what a carried row keeps, or a
+                          // row of a late pass loads
+    uint32_t late_slots;  // late passes: tail slots that no dense op reads
+    int32_t nstaged;      // slots every row's value is read of: 0 .. nstaged-1 (all nslot but in late passes)
     Src keys[SDB_CHAIN_MAX_KEYS];
     int32_t key_min[SDB_CHAIN_MAX_KEYS];
     uint32_t mults[SDB_CHAIN_MAX_KEYS];
@@ -864,31 +861,32 @@ struct Dyn {
     __host__ __device__ static constexpr int key(int) { return kAny; }
 };
 
-// Star join (semi, full, full -> group-by): semi(slot 0); full(slot 1) -> r0;
-// full(slot 2) -> r1; group by (r1, r0), sum slot 3.
+// The late forms (prepare_late), their first ops dense:
+// Star join: semi(slot 0), hit(slot 1) | full(slot 2) -> r1, full(slot 1) ->
+// r0; group by (r1, r0), sum slot 3.
 struct StarBind : Dyn {
     static constexpr bool bound = true;
-    __host__ __device__ static constexpr int a(int i) { return bslot(i); }
-    __host__ __device__ static constexpr int out(int i) { return i == 1 ? 0 : (i == 2 ? 1 : kAny); }
+    __host__ __device__ static constexpr int a(int i) { return i == 3 ? bslot(1) : bslot(i); }
+    __host__ __device__ static constexpr int out(int i) { return i == 2 ? 1 : (i == 3 ? 0 : kAny); }
     __host__ __device__ static constexpr int value() { return bslot(3); }
     __host__ __device__ static constexpr int n_keys() { return 2; }
     __host__ __device__ static constexpr int key(int q) { return q == 0 ? breg(1) : (q == 1 ? breg(0) : kAny); }
 };
 
-// Range filter + join + projection -> group-by (date join): search(slot 0);
-// full(slot 1) -> r0; r1 = slot 2 op slot 0; group by r0, sum r1.
+// Range filter + join + projection -> group-by (date join): search(slot 0),
+// hit(slot 1) | full(slot 1) -> r0, r1 = slot 2 op slot 0; group by r0, sum r1.
 struct DateJoinBind : Dyn {
     static constexpr bool bound = true;
-    __host__ __device__ static constexpr int a(int i) { return bslot(i); }
-    __host__ __device__ static constexpr int b(int i) { return i == 2 ? bslot(0) : kAny; }
-    __host__ __device__ static constexpr int out(int i) { return i == 1 ? 0 : (i == 2 ? 1 : kAny); }
+    __host__ __device__ static constexpr int a(int i) { return i == 0 ? bslot(0) : (i == 3 ? bslot(2) : bslot(1)); }
+    __host__ __device__ static constexpr int b(int i) { return i == 3 ? bslot(0) : kAny; }
+    __host__ __device__ static constexpr int out(int i) { return i == 2 ? 0 : (i == 3 ? 1 : kAny); }
     __host__ __device__ static constexpr int value() { return breg(1); }
     __host__ __device__ static constexpr int n_keys() { return 1; }
     __host__ __device__ static constexpr int key(int q) { return q == 0 ? breg(0) : kAny; }
 };
 
-// Filter-project-sum: search(slot 0), search(slot 1), select(slot 2 cmp
-// literal); r0 = slot 3 op slot 1; sum r0.
+// Filter-project-sum: search(slot 0), search(slot 1) | select(slot 2 cmp
+// literal), r0 = slot 3 op slot 1; sum r0.
 struct FilterSumBind : Dyn {
     static constexpr bool bound = true;
     __host__ __device__ static constexpr int a(int i) { return bslot(i); }
@@ -899,26 +897,28 @@ struct FilterSumBind : Dyn {
 };
 
 // Three full probes with the smallest table pre-tested (SSB flight 3 after
-// prefilter_by_bitmap): bitmap test of slot 1; full(slot 0) -> r0;
-// full(slot 1) -> r1 again for its value; full(slot 2) -> r2; group by
-// (r0, r1, r2), sum slot 3.
+// prefilter_by_bitmap): bitmap test of slot 1, hit(slot 0) | full(slot 1) ->
+// r1, full(slot 2) -> r2, full(slot 0) -> r0; group by (r0, r1, r2), sum slot 3.
 struct Flight3Bind : Dyn {
     static constexpr bool bound = true;
-    __host__ __device__ static constexpr int a(int i) { return i == 1 ? bslot(0) : (i == 3 ? bslot(2) : bslot(1)); }
-    __host__ __device__ static constexpr int out(int i) { return i == 0 ? kAny : i - 1; }
+    __host__ __device__ static constexpr int a(int i)
+    {
+        return i == 1 || i == 4 ? bslot(0) : (i == 3 ? bslot(2) : bslot(1));
+    }
+    __host__ __device__ static constexpr int out(int i) { return i == 2 ? 1 : (i == 3 ? 2 : (i == 4 ? 0 : kAny)); }
     __host__ __device__ static constexpr int value() { return bslot(3); }
     __host__ __device__ static constexpr int n_keys() { return 3; }
     __host__ __device__ static constexpr int key(int q) { return q < 3 ? breg(q) : kAny; }
 };
 
 // Flight 4's second pass (its semi joins run first into the incoming flags):
-// full(slot 0) -> r0; full(slot 1) -> r1; r2 = slot 2 op slot 3; group by
-// (r1, r0), sum r2.
+// hit(slot 0) | full(slot 1) -> r1, full(slot 0) -> r0, r2 = slot 2 op slot 3;
+// group by (r1, r0), sum r2.
 struct Flight4Bind : Dyn {
     static constexpr bool bound = true;
-    __host__ __device__ static constexpr int a(int i) { return bslot(i); }
-    __host__ __device__ static constexpr int b(int i) { return i == 2 ? bslot(3) : kAny; }
-    __host__ __device__ static constexpr int out(int i) { return i; }
+    __host__ __device__ static constexpr int a(int i) { return i == 1 ? bslot(1) : (i == 3 ? bslot(2) : bslot(0)); }
+    __host__ __device__ static constexpr int b(int i) { return i == 3 ? bslot(3) : kAny; }
+    __host__ __device__ static constexpr int out(int i) { return i == 1 ? 1 : (i == 2 ? 0 : (i == 3 ? 2 : kAny)); }
     __host__ __device__ static constexpr int value() { return breg(2); }
     __host__ __device__ static constexpr int n_keys() { return 2; }
     __host__ __device__ static constexpr int key(int q) { return q == 0 ? breg(1) : (q == 1 ? breg(0) : kAny); }
@@ -935,15 +935,15 @@ __host__ __device__ constexpr uint32_t bound_op_bits(int i)
     return code_bit(B::a(i)) | (uses_b ? code_bit(B::b(i)) : 0u);
 }
 
-// The tail and late slot masks of a bound shape (what convert and
-// late_slots_of compute from the launch): the tail is what a compacted row
-// keeps -- the slots the ops after the first read (from the first on when
-// the rows are compacted on their incoming flags, SPLIT 0).
+// The tail and late slot masks of a bound shape (what prepare_late computes
+// from the launch): the tail is what a compacted row keeps -- the slots that
+// the ops from SPLIT on and the terminal read --, the late ones of it those
+// that no op before SPLIT reads.
 template <class B, int TERM, int SPLIT, int... KS>
 __host__ __device__ constexpr uint32_t bound_tail()
 {
     uint32_t m = 0;
-    for (int i = SPLIT == 0 ? 0 : 1; i < (int)sizeof...(KS); i++) m |= bound_op_bits<B, KS...>(i);
+    for (int i = SPLIT; i < (int)sizeof...(KS); i++) m |= bound_op_bits<B, KS...>(i);
     if (TERM != T_FLAGS) m |= code_bit(B::value());
     for (int q = 0; q < B::n_keys(); q++) m |= code_bit(B::key(q));
     return m;
@@ -952,7 +952,7 @@ template <class B, int TERM, int SPLIT, int... KS>
 __host__ __device__ constexpr uint32_t bound_late()
 {
     uint32_t e = 0;
-    for (int i = 0; i <= SPLIT && i < (int)sizeof...(KS); i++) e |= bound_op_bits<B, KS...>(i);
+    for (int i = 0; i < SPLIT && i < (int)sizeof...(KS); i++) e |= bound_op_bits<B, KS...>(i);
     return bound_tail<B, TERM, SPLIT, KS...>() & ~e;
 }
 
@@ -1065,12 +1065,12 @@ __device__ __forceinline__ void store4(int32_t *col, uint64_t base, const int32_
         if ((mask >> k) & 1u) col[base + k] = v[k];
 }
 
-template <int K, int A, int BB, int OUT, int NREGS, int IT>
-__device__ __forceinline__ void step(const Op &op, State<NREGS, IT> &S)
+template <int K, int A, int BB, int OUT, class StateT>
+__device__ __forceinline__ void step(const Op &op, StateT &S)
 {
-    constexpr int kItems = IT;
+    constexpr int kItems = StateT::kIt;
     int32_t a[kItems], b[kItems];
-    if (K == SDB_OP_SELECT || K == SDB_OP_SEARCH_RANGE || K == SDB_OP_SEARCH_POINTS) {
+    if constexpr (K == SDB_OP_SELECT || K == SDB_OP_SEARCH_RANGE || K == SDB_OP_SEARCH_POINTS) {
         const bool and_op = op.logic == SDB_AND;
         if (and_op && S.live == 0) return;
         const uint32_t need = and_op ? S.live : S.valid;
@@ -1086,7 +1086,7 @@ __device__ __forceinline__ void step(const Op &op, State<NREGS, IT> &S)
             m |= (uint32_t)c << k;
         }
         S.live = sdb::logical4(op.logic, S.live, m & need) & S.valid;
-    } else if (K == SDB_OP_SEMI_PROBE) {
+    } else if constexpr (K == SDB_OP_SEMI_PROBE) {
         if (S.live == 0) return;
         fetch4c<A>(op.a, S, a);
         const uint8_t *ht = static_cast<const uint8_t *>(op.ht);
@@ -1111,7 +1111,21 @@ __device__ __forceinline__ void step(const Op &op, State<NREGS, IT> &S)
             for (int k = 0; k < kItems; k++) m |= (uint32_t)(h[k] != 0) << k;
         }
         S.live &= m;
-    } else if (K == SDB_OP_FULL_PROBE) {
+    } else if constexpr (K == K_HIT) {  // the live rows' entries, every read in flight together
+        if (S.live == 0) return;
+        fetch4c<A>(op.a, S, a);
+        const int2 *ht = static_cast<const int2 *>(op.ht);
+        int32_t x[kItems];
+#pragma unroll
+        for (int k = 0; k < kItems; k++) {
+            x[k] = 0;
+            if (((S.live >> k) & 1u) && in_range(a[k], op.lo, op.hi)) x[k] = __ldg(&ht[(uint32_t)a[k] - (uint32_t)op.lo].x);
+        }
+        uint32_t m = 0;
+#pragma unroll
+        for (int k = 0; k < kItems; k++) m |= (uint32_t)(x[k] == 1) << k;
+        S.live &= m;
+    } else if constexpr (K == SDB_OP_FULL_PROBE) {
         if (S.live == 0) return;
         fetch4c<A>(op.a, S, a);
         const int2 *ht = static_cast<const int2 *>(op.ht);
@@ -1132,7 +1146,7 @@ __device__ __forceinline__ void step(const Op &op, State<NREGS, IT> &S)
         S.live = m;
         set_regs_c<OUT>(S, op.out_reg, b, m);
         if (op.out_col && m) store4(op.out_col, S.base, b, m);
-    } else if (K == SDB_OP_BINOP) {
+    } else if constexpr (K == SDB_OP_BINOP) {
         if (S.live == 0) return;
         fetch4c<A>(op.a, S, a);
         fetch4c<BB>(op.b, S, b);
@@ -1140,7 +1154,7 @@ __device__ __forceinline__ void step(const Op &op, State<NREGS, IT> &S)
         for (int k = 0; k < kItems; k++) a[k] = sdb::binop(a[k], b[k], op.bin);
         set_regs_c<OUT>(S, op.out_reg, a, S.live);
         if (op.out_col) store4(op.out_col, S.base, a, S.live);
-    } else if (K == SDB_OP_FILL) {
+    } else if constexpr (K == SDB_OP_FILL) {
 #pragma unroll
         for (int k = 0; k < kItems; k++) a[k] = op.a.lit;
         set_regs_c<OUT>(S, op.out_reg, a, S.valid);
@@ -1148,8 +1162,8 @@ __device__ __forceinline__ void step(const Op &op, State<NREGS, IT> &S)
     }
 }
 
-template <class B, int NREGS, int BEGIN, int... KS, int IT, int... IS>
-__device__ __forceinline__ void run_steps(const Launch &L, State<NREGS, IT> &S, std::integer_sequence<int, IS...>)
+template <class B, int BEGIN, int... KS, class StateT, int... IS>
+__device__ __forceinline__ void run_steps(const Launch &L, StateT &S, std::integer_sequence<int, IS...>)
 {
     constexpr int kinds[] = {KS...};
     (step<kinds[BEGIN + IS], B::a(BEGIN + IS), B::b(BEGIN + IS), B::out(BEGIN + IS)>(L.ops[BEGIN + IS], S), ...);
@@ -1325,8 +1339,8 @@ __device__ __forceinline__ void group_row(const LaunchT &L, uint32_t *s_key, uin
 // SPLIT = number of ops run on 4-row groups; the rest run on the compacted
 // rows.  SPLIT == sizeof...(KS) + 1 means no compaction (all ops dense, which
 // also serves SDB_TERM_FLAGS).
-template <int STAGES, int CARRY>
-__host__ __device__ constexpr int dense_min_blocks() { return CARRY == 3 ? 5 : (STAGES >= 3 ? 3 : 5); }
+template <int STAGES>
+__host__ __device__ constexpr int dense_min_blocks() { return STAGES >= 3 ? 3 : 5; }
 
 // ---- pieces shared by the single-chain pass and the batched pass ----------
 
@@ -1485,22 +1499,12 @@ __device__ __forceinline__ VRow<NREGS> take_row(const VRow<NREGS> &R, const uint
 }
 
 // The ops after the first row-per-lane op and the terminal, for the rows of
-// a level-2 group (lane j: row j while F.live).  CARRY 3 first loads the late
-// slots of each live row from its row number.
+// a level-2 group (lane j: row j while F.live).
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_run(const Launch &L, VRow<NREGS> &F, const uint32_t *s_bits, uint32_t *s_key,
                                            uint32_t *s_sum, bool direct, uint64_t &acc)
 {
     constexpr int N = sizeof...(KS);
-    if constexpr (CARRY == 3) {
-        const uint32_t late = B::bound ? bound_late<B, TERM, SPLIT, KS...>() : L.late_slots;
-        if (F.live) {
-            if (late & 1u) F.v0 = __ldg(L.slot[0] + (uint32_t)F.v0);
-            if (late & 2u) F.v1 = __ldg(L.slot[1] + (uint32_t)F.v1);
-            if (late & 4u) F.v2 = __ldg(L.slot[2] + (uint32_t)F.v2);
-            if (late & 8u) F.v3 = __ldg(L.slot[3] + (uint32_t)F.v3);
-        }
-    }
     run_steps1<B, NREGS, SPLIT + 1, KS...>(L, F, s_bits, std::make_integer_sequence<int, N - SPLIT - 1>{});
     finish_row<TERM, B>(L, F, s_key, s_sum, direct, acc);
 }
@@ -1540,12 +1544,12 @@ __device__ __forceinline__ void level2_push(const Launch &L, const VRow<NREGS> &
     __syncwarp();  // every lane has read the list before it is written again
 }
 
-// Whether CARRY 2 or 3 uses the second level: there are ops after the first
+// Whether CARRY 2 uses the second level: there are ops after the first
 // row-per-lane op.
 template <int SPLIT, int... KS>
 __host__ __device__ constexpr bool use_level2(int carry)
 {
-    return carry >= 2 && SPLIT + 1 < (int)sizeof...(KS);
+    return carry == 2 && SPLIT + 1 < (int)sizeof...(KS);
 }
 
 // The first row-per-lane op and then the second level, for one group.
@@ -1592,26 +1596,16 @@ __device__ __forceinline__ void drain_carry(const Launch &L, uint32_t &carry, co
     __syncwarp();
 }
 
-// What a compacted row keeps of slot s: its staged value when a later op
-// reads the slot, or (CARRY 3, late slot) its row number, row0 + r.
-template <int CARRY, class B, int TERM, int SPLIT, int SL, int... KS>
-__device__ __forceinline__ int32_t tail_value(const Launch &L, const int32_t *ws, uint32_t r, uint64_t row0)
+// What a compacted row keeps of slot SL: its staged value when a later op reads
+// the slot.
+template <int SL>
+__device__ __forceinline__ int32_t tail_value(const Launch &L, const int32_t *ws, uint32_t r)
 {
-    if constexpr (B::bound) {
-        constexpr uint32_t tail = bound_tail<B, TERM, SPLIT, KS...>();
-        constexpr uint32_t late = CARRY == 3 ? bound_late<B, TERM, SPLIT, KS...>() : 0u;
-        if constexpr (!((tail >> SL) & 1u)) return 0;
-        else if constexpr ((late >> SL) & 1u) return (int32_t)(uint32_t)(row0 + r);
-        else return ws[SL * items_of<CARRY>() * kThreads + r];
-    } else {
-        if (!((L.tail_slots >> SL) & 1u)) return 0;
-        if (CARRY == 3 && ((L.late_slots >> SL) & 1u)) return (int32_t)(uint32_t)(row0 + r);
-        return ws[SL * items_of<CARRY>() * kThreads + r];
-    }
+    return (L.tail_slots >> SL) & 1u ? ws[SL * kItems * kThreads + r] : 0;
 }
 
 template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
-__device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of<CARRY>()> &S, const int4 *s_buf, int st,
+__device__ __forceinline__ void tile_body(const Launch &L, State<NREGS> &S, const int4 *s_buf, int st,
                                           uint64_t tile,
                                           uint8_t *s_list, uint32_t *s_key, uint32_t *s_sum,
                                           const uint32_t *s_bits, bool direct, uint64_t &acc, uint32_t &carry,
@@ -1620,9 +1614,8 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
     constexpr int N = sizeof...(KS);
     constexpr bool kCompact = SPLIT <= N;
     constexpr int kDenseOps = kCompact ? SPLIT : N;
-    constexpr int kItems = items_of<CARRY>(), kQ = kItems / 4;
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    constexpr int SS = stage_slots<CARRY>();
+    constexpr int SS = kSlots;
     S.stage = &s_buf[(st * SS * kThreads + threadIdx.x) * kQ];
     S.base = tile + (uint64_t)kItems * threadIdx.x;
     if (S.base + kItems <= L.n) {
@@ -1634,20 +1627,14 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
     }
     if (L.flags_in && S.valid) {
         uint32_t m = 0;
-        if (kItems == 8 && S.valid == 0xffu && sdb::aligned(L.flags_in, 8)) {  // 8 flags in one load
-            const uint64_t f = *reinterpret_cast<const uint64_t *>(L.flags_in + S.base);
 #pragma unroll
-            for (int k = 0; k < 8; k++) m |= (uint32_t)(((f >> (8 * k)) & 0xffu) != 0) << k;
-        } else {
-#pragma unroll
-            for (int k = 0; k < kItems; k++)
-                if ((S.valid >> k) & 1u) m |= (uint32_t)(L.flags_in[S.base + k] != 0) << k;
-        }
+        for (int k = 0; k < kItems; k++)
+            if ((S.valid >> k) & 1u) m |= (uint32_t)(L.flags_in[S.base + k] != 0) << k;
         S.live = m;
     } else {
         S.live = S.valid;
     }
-    run_steps<B, NREGS, 0, KS...>(L, S, std::make_integer_sequence<int, kDenseOps>{});
+    run_steps<B, 0, KS...>(L, S, std::make_integer_sequence<int, kDenseOps>{});
 
     if constexpr (kCompact) {
         // warp prefix sum of the live-row counts
@@ -1670,7 +1657,6 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
             // entries 0 .. carry-1 are the carried rows (entry j in lane j),
             // then this tile's survivors
             const uint32_t avail = carry + total;
-            const uint64_t row0 = tile + (uint64_t)warp * 32 * kItems;  // row of the warp's staged row 0
             auto entry = [&](uint32_t idx) {
                 VRow<NREGS> R;
                 if (idx < carry) {  // only in the first group: idx == lane
@@ -1680,10 +1666,10 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
                     R.v3 = ce.w;
                 } else {
                     const uint32_t r = list[idx - carry];
-                    R.v0 = tail_value<CARRY, B, TERM, SPLIT, 0, KS...>(L, ws, r, row0);
-                    R.v1 = tail_value<CARRY, B, TERM, SPLIT, 1, KS...>(L, ws, r, row0);
-                    R.v2 = tail_value<CARRY, B, TERM, SPLIT, 2, KS...>(L, ws, r, row0);
-                    R.v3 = tail_value<CARRY, B, TERM, SPLIT, 3, KS...>(L, ws, r, row0);
+                    R.v0 = tail_value<0>(L, ws, r);
+                    R.v1 = tail_value<1>(L, ws, r);
+                    R.v2 = tail_value<2>(L, ws, r);
+                    R.v3 = tail_value<3>(L, ws, r);
                 }
                 R.live = true;
                 return R;
@@ -1699,10 +1685,10 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS, items_of
             const uint32_t rem = avail - b;
             if (lane < rem && b + lane >= carry) {  // carry a survivor of this tile
                 const uint32_t r = list[b + lane - carry];
-                ce.x = tail_value<CARRY, B, TERM, SPLIT, 0, KS...>(L, ws, r, row0);
-                ce.y = tail_value<CARRY, B, TERM, SPLIT, 1, KS...>(L, ws, r, row0);
-                ce.z = tail_value<CARRY, B, TERM, SPLIT, 2, KS...>(L, ws, r, row0);
-                ce.w = tail_value<CARRY, B, TERM, SPLIT, 3, KS...>(L, ws, r, row0);
+                ce.x = tail_value<0>(L, ws, r);
+                ce.y = tail_value<1>(L, ws, r);
+                ce.z = tail_value<2>(L, ws, r);
+                ce.w = tail_value<3>(L, ws, r);
             }
             carry = rem;
             __syncwarp();
@@ -1781,22 +1767,21 @@ __device__ __forceinline__ void block_flush(const LaunchT &L, uint32_t *s_key, u
 }
 
 template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
-__global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>()) k_dense(const __grid_constant__ Launch L)
+__global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES>()) k_dense(const __grid_constant__ Launch L)
 {
     constexpr int kStages = STAGES;
     constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
-    constexpr int kItems = items_of<CARRY>(), kQ = kItems / 4;
-    constexpr int SS = stage_slots<CARRY>();
+    constexpr int SS = kSlots;
     extern __shared__ int4 s_buf[];  // [kStages][SS][kThreads][kQ], then the semi-join bitmap
     __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
     __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kDenseCap : 1];
     __shared__ uint8_t s_list[kCompact ? kThreads * kItems : 1];  // per warp: 32 x kItems row offsets
     __shared__ uint64_t s_part[kThreads / 32];
-    __shared__ uint8_t s_l2src[CARRY >= 2 ? kThreads : 1];
+    __shared__ uint8_t s_l2src[CARRY == 2 ? kThreads : 1];
     uint32_t carry = 0;  // rows the warp carries (warp-uniform)
     int4 ce = make_int4(0, 0, 0, 0);
     Level2<NREGS> Q;
-    Q.src = s_l2src + (CARRY >= 2 ? (threadIdx.x & ~31u) : 0u);
+    Q.src = s_l2src + (CARRY == 2 ? (threadIdx.x & ~31u) : 0u);
     const bool direct = L.P <= kDenseCap;
     uint32_t *s_bits = reinterpret_cast<uint32_t *>(s_buf + kStages * SS * kThreads * kQ);
     constexpr uint64_t kTile = (uint64_t)kThreads * kItems;
@@ -1834,89 +1819,252 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>()) k
     block_flush<TERM>(L, s_key, s_sum, s_part, acc);
 }
 
+// ---------------------------------------------------------------- late passes
+// The pass of the hot shapes.  Ops before SPLIT run on 8 rows per thread whose
+// (at most two) columns a thread reads straight into registers, a tile ahead;
+// the rows that are left, a few percent, are queued by row number per warp,
+// and whenever 32 are pending they load the columns that the later ops and the
+// terminal read (only the sectors holding such rows) and run them one row per
+// lane.
+//
+// Registers and not a copy ring for the tile ahead: the passes spend their
+// time on random reads of join tables, and what an SM can have in flight or
+// find again there is bounded by its L1, the part of its 256 KB that shared
+// memory leaves.  Plain loads and not evict-first ones: the columns' sectors are read
+// again by row number.  Plans at 120 M rows, star join / date join /
+// filter-project-sum: 300 / 341 / 272 us with a 32 KB ring, compaction after
+// the first op and a second compaction level (the former pass; with its L1
+// squeezed to 28 KB by the carveout the star join took 330); 281 / 354 / 295
+// this way with evict-first loads; 275 / 282 / 254 as it is.  Five blocks per SM (51 registers): 264 /
+// 266 / 266, but 104 against 100 for the star join at 30 M rows.
+constexpr int kLateItems = 8;
+constexpr int kLateSlots = 2;
+
+struct LateState {
+    static constexpr int kIt = kLateItems;
+    int4 cur[kLateSlots][kIt / 4];  // this thread's rows of the tile
+    const uint32_t *bits;
+    uint64_t base;
+    uint32_t valid, live;
+};
+
+template <int C>
+__device__ __forceinline__ void fetch4c(const Src &s, const LateState &S, int32_t (&v)[kLateItems])
+{
+    if constexpr (C == kLitCode) {
+#pragma unroll
+        for (int k = 0; k < kLateItems; k++) v[k] = s.lit;
+    } else {
+        static_assert(C == kAny || C < kLateSlots, "a dense op of a late pass reads a staged slot");
+        const bool one = C == kAny ? s.idx == 1 : C == 1;
+#pragma unroll
+        for (int q = 0; q < kLateItems / 4; q++) {
+            const int4 x = one ? S.cur[1][q] : S.cur[0][q];
+            v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+        }
+        if (C == kAny && s.src == 2) {
+#pragma unroll
+            for (int k = 0; k < kLateItems; k++) v[k] = s.lit;
+        }
+    }
+}
+
+// Reads the thread's rows of the staged columns (rows past the end: zero).
+template <class B, int SPLIT, int... KS>
+__device__ __forceinline__ void late_load(const Launch &L, uint64_t tile, int4 (&v)[kLateSlots][kLateItems / 4])
+{
+    uint32_t early = 0;  // a bound pass knows how many columns there are
+    for (int i = 0; i < SPLIT; i++) early |= B::bound ? bound_op_bits<B, KS...>(i) : 0u;
+    const int staged = B::bound ? ((early >> 1) & 1u ? 2 : 1) : L.nstaged;
+#pragma unroll
+    for (int s = 0; s < kLateSlots; s++) {
+        if (s >= staged) continue;
+        const int32_t *col = L.slot[s];
+#pragma unroll
+        for (int q = 0; q < kLateItems / 4; q++) {
+            const uint64_t r = tile + (uint64_t)kLateItems * threadIdx.x + 4 * q;
+            if (r + 4 <= L.n) {
+                v[s][q] = __ldg(reinterpret_cast<const int4 *>(col + r));
+            } else {
+                v[s][q] = make_int4(r < L.n ? col[r] : 0, r + 1 < L.n ? col[r + 1] : 0, r + 2 < L.n ? col[r + 2] : 0, 0);
+            }
+        }
+    }
+}
+
+// One row per lane: the columns it needs by its row number, all together,
+// then the ops from SPLIT on and the terminal.
+template <int TERM, class B, int NREGS, int SPLIT, int... KS>
+__device__ __forceinline__ void late_rows(const Launch &L, uint32_t row, bool live, const uint32_t *s_bits, uint32_t *s_key,
+                                          uint32_t *s_sum, bool direct, uint64_t &acc)
+{
+    const uint32_t tail = B::bound ? bound_tail<B, TERM, SPLIT, KS...>() : L.tail_slots;
+    VRow<NREGS> R;
+    R.live = live;
+    R.v0 = R.v1 = R.v2 = R.v3 = 0;
+    if (live) {
+        if (tail & 1u) R.v0 = __ldg(L.slot[0] + row);
+        if (tail & 2u) R.v1 = __ldg(L.slot[1] + row);
+        if (tail & 4u) R.v2 = __ldg(L.slot[2] + row);
+        if (tail & 8u) R.v3 = __ldg(L.slot[3] + row);
+    }
+    sparse_row<TERM, B, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
+}
+
+// One tile of one chain: S.cur holds its columns.  `queued` of the warp's 64
+// queue entries are pending (fewer than 32 between calls).
+template <int TERM, class B, int NREGS, int SPLIT, int... KS>
+__device__ __forceinline__ void late_tile(const Launch &L, LateState &S, uint64_t tile, uint32_t *queue, uint32_t &queued,
+                                          const uint32_t *s_bits, uint32_t *s_key, uint32_t *s_sum, bool direct, uint64_t &acc)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    S.bits = s_bits;
+    S.base = tile + (uint64_t)kLateItems * threadIdx.x;
+    S.valid = (1u << kLateItems) - 1u;
+    if (S.base + kLateItems > L.n) S.valid = S.base < L.n ? (1u << (uint32_t)(L.n - S.base)) - 1u : 0u;
+    S.live = S.valid;
+    if (L.flags_in && S.valid) {
+        uint32_t m = 0;
+        if (S.valid == 0xffu && sdb::aligned(L.flags_in, 8)) {  // 8 flags in one load
+            const uint64_t f = *reinterpret_cast<const uint64_t *>(L.flags_in + S.base);
+#pragma unroll
+            for (int k = 0; k < kLateItems; k++) m |= (uint32_t)(((f >> (8 * k)) & 0xffu) != 0) << k;
+        } else {
+#pragma unroll
+            for (int k = 0; k < kLateItems; k++)
+                if ((S.valid >> k) & 1u) m |= (uint32_t)(L.flags_in[S.base + k] != 0) << k;
+        }
+        S.live = m;
+    }
+    run_steps<B, 0, KS...>(L, S, std::make_integer_sequence<int, SPLIT>{});
+    // queue the rows, one of each lane at a time (their order does not matter:
+    // sums and group-by slots)
+    uint32_t live = S.live;
+    for (;;) {
+        const unsigned m = __ballot_sync(0xffffffffu, live != 0);
+        if (m == 0) break;
+        if (live) {
+            queue[queued + __popc(m & ((1u << lane) - 1u))] = (uint32_t)S.base + (uint32_t)__ffs(live) - 1u;
+            live &= live - 1;
+        }
+        queued += __popc(m);
+        __syncwarp();
+        if (queued >= 32) {
+            queued -= 32;
+            const uint32_t row = queue[queued + lane];
+            __syncwarp();  // read before the queue grows again
+            late_rows<TERM, B, NREGS, SPLIT, KS...>(L, row, true, s_bits, s_key, s_sum, direct, acc);
+        }
+    }
+}
+
+// What is left in the queue (at the end of a block's rows of a chain).
+template <int TERM, class B, int NREGS, int SPLIT, int... KS>
+__device__ __forceinline__ void late_drain(const Launch &L, const uint32_t *queue, uint32_t &queued, const uint32_t *s_bits,
+                                           uint32_t *s_key, uint32_t *s_sum, bool direct, uint64_t &acc)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    if (queued)
+        late_rows<TERM, B, NREGS, SPLIT, KS...>(L, lane < queued ? queue[lane] : 0u, lane < queued, s_bits, s_key, s_sum,
+                                                direct, acc);
+    queued = 0;
+    __syncwarp();
+}
+
+constexpr int kLateBlocks = 4;  // resident blocks per SM (64 registers a thread)
+
+template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+__global__ void __launch_bounds__(kThreads, kLateBlocks) k_late(const __grid_constant__ Launch L)
+{
+    extern __shared__ uint32_t s_bits[];  // the semi-join bitmap
+    __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
+    __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kDenseCap : 1];
+    __shared__ uint32_t s_queue[kThreads / 32][64];  // per warp: row numbers
+    __shared__ uint64_t s_part[kThreads / 32];
+    constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
+    const uint64_t stride = (uint64_t)gridDim.x * kTile;
+    uint64_t tile = (uint64_t)blockIdx.x * kTile;
+    LateState S;
+    int4 next[kLateSlots][kLateItems / 4] = {};
+    // the first tile's reads are in flight while the group table and the
+    // bitmap are set up
+    late_load<B, SPLIT, KS...>(L, tile, next);
+    group_table_reset<TERM>(s_key, s_sum);
+    stage_bitmap(L, s_bits);
+    if (TERM == T_GROUP || L.bitmap_ht) __syncthreads();
+    const bool direct = L.P <= kDenseCap;
+    uint64_t acc = 0;
+    uint32_t queued = 0;
+    uint32_t *queue = s_queue[threadIdx.x >> 5];
+    for (; tile < L.n; tile += stride) {
+#pragma unroll
+        for (int s = 0; s < kLateSlots; s++)
+#pragma unroll
+            for (int q = 0; q < kLateItems / 4; q++) S.cur[s][q] = next[s][q];
+        late_load<B, SPLIT, KS...>(L, tile + stride, next);
+        late_tile<TERM, B, NREGS, SPLIT, KS...>(L, S, tile, queue, queued, s_bits, s_key, s_sum, direct, acc);
+    }
+    late_drain<TERM, B, NREGS, SPLIT, KS...>(L, queue, queued, s_bits, s_key, s_sum, direct, acc);
+    block_flush<TERM>(L, s_key, s_sum, s_part, acc);
+}
+
 // Paired pass: two chains of one bound shape whose staged slots are the same
 // columns over the same rows (two plans of a batch that scan the same fact
-// rows with their own literals and tables).  Each tile is copied into the
-// ring once and both chains run on it, each with its own group table,
-// bitmap, carried rows and second-level rows; late columns are each chain's
-// own.  The host checks that the staged slots, row count and incoming flags
-// (none) agree.
+// rows with their own literals and tables).  Each tile is read once and both
+// chains run on it, each with its own group table, bitmap and queued rows;
+// late columns are each chain's own.  The host checks that the staged slots,
+// row count and incoming flags (none) agree.
 constexpr int kPair = 2;
 struct LaunchPair {
     Launch L[kPair];
-    uint32_t bits_off[kPair];  // each chain's bitmap: its first word after the ring
+    uint32_t bits_off[kPair];  // each chain's bitmap: its first word
 };
 
-template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
-__global__ void __launch_bounds__(kThreads, 4) k_dense_pair(const __grid_constant__ LaunchPair P)
+template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+__global__ void __launch_bounds__(kThreads, kLateBlocks) k_late_pair(const __grid_constant__ LaunchPair P)
 {
-    static_assert(B::bound && CARRY == 3, "the paired pass runs the bound carry-3 shapes");
-    constexpr int kStages = STAGES;
-    constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
-    constexpr int kItems = items_of<CARRY>(), kQ = kItems / 4;
-    constexpr int SS = stage_slots<CARRY>();
-    extern __shared__ int4 s_buf[];  // [kStages][SS][kThreads][kQ], then the chains' bitmaps
+    static_assert(B::bound, "the paired pass runs the bound shapes");
+    extern __shared__ uint32_t s_bitmaps[];
     __shared__ uint32_t s_key[kPair][TERM == T_GROUP ? kDenseCap : 1];
     __shared__ uint32_t s_sum[kPair][TERM == T_GROUP ? 2 * kDenseCap : 1];
-    __shared__ uint8_t s_list[kCompact ? kThreads * kItems : 1];  // reused by the chains in turn
+    __shared__ uint32_t s_queue[kPair][kThreads / 32][64];
     __shared__ uint64_t s_part[kThreads / 32];
-    __shared__ uint8_t s_l2src[kPair][kThreads];
     const Launch &L0 = P.L[0];  // the staged slots, row count and tiles are L0's (and L1's)
-    uint32_t carry[kPair];
-    int4 ce[kPair];
-    Level2<NREGS> Q[kPair];
+    constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
+    const uint64_t stride = (uint64_t)gridDim.x * kTile;
+    uint64_t tile = (uint64_t)blockIdx.x * kTile;
+    LateState S;
+    int4 next[kLateSlots][kLateItems / 4] = {};
+    late_load<B, SPLIT, KS...>(L0, tile, next);
+    uint32_t queued[kPair];
     bool direct[kPair];
     uint64_t acc[kPair];
     uint32_t *s_bits[kPair];
-    uint32_t *ring_end = reinterpret_cast<uint32_t *>(s_buf + kStages * SS * kThreads * kQ);
 #pragma unroll
     for (int c = 0; c < kPair; c++) {
-        carry[c] = 0;
-        ce[c] = make_int4(0, 0, 0, 0);
-        Q[c].src = s_l2src[c] + (threadIdx.x & ~31u);
+        queued[c] = 0;
         direct[c] = P.L[c].P <= kDenseCap;
         acc[c] = 0;
-        s_bits[c] = ring_end + P.bits_off[c];
-    }
-    constexpr uint64_t kTile = (uint64_t)kThreads * kItems;
-    const uint64_t stride = (uint64_t)gridDim.x * kTile;
-    uint64_t tile = (uint64_t)blockIdx.x * kTile;
-#pragma unroll
-    for (int p = 0; p < kStages - 1; p++)
-        issue_tile<kStages, SS, kItems>(L0.slot, L0.nstaged, L0.n, s_buf, p, tile + p * stride);
-#pragma unroll
-    for (int c = 0; c < kPair; c++) {
+        s_bits[c] = s_bitmaps + P.bits_off[c];
         group_table_reset<TERM>(s_key[c], s_sum[c]);
         stage_bitmap(P.L[c], s_bits[c]);
     }
     __syncthreads();
-
-    State<NREGS, kItems> S;
-#pragma unroll
-    for (int r = 0; r < NREGS; r++)
-#pragma unroll
-        for (int k = 0; k < kItems; k++) S.reg[r][k] = 0;
-
-    int st = 0;
     for (; tile < L0.n; tile += stride) {
-        issue_tile<kStages, SS, kItems>(L0.slot, L0.nstaged, L0.n, s_buf, (st + kStages - 1) % kStages,
-                                        tile + (kStages - 1) * stride);
-        cp_async_wait<kStages - 1>();
 #pragma unroll
-        for (int c = 0; c < kPair; c++) {
-            S.bits = s_bits[c];
-            tile_body<TERM, B, NREGS, SPLIT, CARRY, KS...>(P.L[c], S, s_buf, st, tile, s_list, s_key[c], s_sum[c],
-                                                           s_bits[c], direct[c], acc[c], carry[c], ce[c], Q[c]);
-        }
-        st = (st + 1) % kStages;
+        for (int s = 0; s < kLateSlots; s++)
+#pragma unroll
+            for (int q = 0; q < kLateItems / 4; q++) S.cur[s][q] = next[s][q];
+        late_load<B, SPLIT, KS...>(L0, tile + stride, next);
+#pragma unroll
+        for (int c = 0; c < kPair; c++)
+            late_tile<TERM, B, NREGS, SPLIT, KS...>(P.L[c], S, tile, s_queue[c][threadIdx.x >> 5], queued[c], s_bits[c],
+                                                    s_key[c], s_sum[c], direct[c], acc[c]);
     }
-    cp_async_wait<0>();
-#pragma unroll
-    for (int c = 0; c < kPair; c++)
-        drain_carry<TERM, B, NREGS, SPLIT, CARRY, KS...>(P.L[c], carry[c], ce[c], Q[c], s_bits[c], s_key[c], s_sum[c],
-                                                         direct[c], acc[c]);
 #pragma unroll
     for (int c = 0; c < kPair; c++) {
+        late_drain<TERM, B, NREGS, SPLIT, KS...>(P.L[c], s_queue[c][threadIdx.x >> 5], queued[c], s_bits[c], s_key[c],
+                                                 s_sum[c], direct[c], acc[c]);
         if (c) __syncthreads();  // the first flush has read s_part
         block_flush<TERM>(P.L[c], s_key[c], s_sum[c], s_part, acc[c]);
     }
@@ -1937,18 +2085,17 @@ struct Span {
 // Within a span the tiles go through the same cp.async ring as the
 // single-chain pass.
 template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
-__global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>())
+__global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES>())
     k_batch(const Launch *__restrict__ launches, const Span *__restrict__ spans, uint32_t n_spans,
             uint32_t *__restrict__ head)
 {
-    __shared__ uint8_t s_l2src[CARRY >= 2 ? kThreads : 1];
+    __shared__ uint8_t s_l2src[CARRY == 2 ? kThreads : 1];
     uint32_t carry = 0;
     int4 ce = make_int4(0, 0, 0, 0);
     Level2<NREGS> Q;
-    Q.src = s_l2src + (CARRY >= 2 ? (threadIdx.x & ~31u) : 0u);
+    Q.src = s_l2src + (CARRY == 2 ? (threadIdx.x & ~31u) : 0u);
     constexpr int kStages = STAGES;
     constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
-    constexpr int kItems = items_of<CARRY>(), kQ = kItems / 4;
     constexpr uint64_t kTile = (uint64_t)kThreads * kItems;
     extern __shared__ int4 s_buf[];
     __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
@@ -1957,7 +2104,7 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>())
     __shared__ uint64_t s_part[kThreads / 32];
     __shared__ Launch s_L;
     __shared__ uint32_t s_next;
-    constexpr int SS = stage_slots<CARRY>();
+    constexpr int SS = kSlots;
     uint32_t *s_bits = reinterpret_cast<uint32_t *>(s_buf + kStages * SS * kThreads * kQ);
 
     State<NREGS, kItems> S;
@@ -2016,6 +2163,62 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES, CARRY>())
     if (cur != ~0u) block_flush<TERM>(s_L, s_key, s_sum, s_part, acc);
 }
 
+// The batched pass over chains of one late shape: spans pulled as in k_batch,
+// each span's tiles as in k_late.
+template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+__global__ void __launch_bounds__(kThreads, kLateBlocks)
+    k_batch_late(const Launch *__restrict__ launches, const Span *__restrict__ spans, uint32_t n_spans,
+                 uint32_t *__restrict__ head)
+{
+    extern __shared__ uint32_t s_bits[];
+    __shared__ uint32_t s_key[TERM == T_GROUP ? kDenseCap : 1];
+    __shared__ uint32_t s_sum[TERM == T_GROUP ? 2 * kDenseCap : 1];
+    __shared__ uint32_t s_queue[kThreads / 32][64];
+    __shared__ uint64_t s_part[kThreads / 32];
+    __shared__ Launch s_L;
+    __shared__ uint32_t s_next;
+    constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
+    LateState S;
+    uint64_t acc = 0;
+    uint32_t queued = 0, cur = ~0u;
+    uint32_t *queue = s_queue[threadIdx.x >> 5];
+    for (;;) {
+        if (threadIdx.x == 0) s_next = atomicAdd(head, 1u);
+        __syncthreads();
+        const uint32_t sp = s_next;
+        __syncthreads();  // every thread has read s_next before thread 0 writes it again
+        if (sp >= n_spans) break;
+        const Span span = spans[sp];
+        if (span.chain != cur) {
+            if (cur != ~0u) block_flush<TERM>(s_L, s_key, s_sum, s_part, acc);
+            __syncthreads();
+            const uint32_t *src = reinterpret_cast<const uint32_t *>(&launches[span.chain]);
+            uint32_t *dst = reinterpret_cast<uint32_t *>(&s_L);
+            for (uint32_t w = threadIdx.x; w < sizeof(Launch) / 4; w += blockDim.x) dst[w] = src[w];
+            group_table_reset<TERM>(s_key, s_sum);
+            __syncthreads();
+            stage_bitmap(s_L, s_bits);
+            __syncthreads();
+            cur = span.chain;
+        }
+        const bool direct = s_L.P <= kDenseCap;
+        int4 next[kLateSlots][kLateItems / 4] = {};
+        late_load<B, SPLIT, KS...>(s_L, (uint64_t)span.t0 * kTile, next);
+        for (uint32_t t = span.t0; t < span.t1; t++) {
+#pragma unroll
+            for (int s = 0; s < kLateSlots; s++)
+#pragma unroll
+                for (int q = 0; q < kLateItems / 4; q++) S.cur[s][q] = next[s][q];
+            if (t + 1 < span.t1) late_load<B, SPLIT, KS...>(s_L, (uint64_t)(t + 1) * kTile, next);
+            late_tile<TERM, B, NREGS, SPLIT, KS...>(s_L, S, (uint64_t)t * kTile, queue, queued, s_bits, s_key, s_sum, direct,
+                                                    acc);
+        }
+        // queued rows belong to this span's chain: run them before the next pull
+        late_drain<TERM, B, NREGS, SPLIT, KS...>(s_L, queue, queued, s_bits, s_key, s_sum, direct, acc);
+    }
+    if (cur != ~0u) block_flush<TERM>(s_L, s_key, s_sum, s_part, acc);
+}
+
 // Launches of the specialised passes, and of those the bound ones (host
 // counters, read by sdb_fused_launch_counts).
 std::atomic<uint64_t> g_dense_launches{0}, g_bound_launches{0};
@@ -2024,7 +2227,7 @@ template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int...
 int launch_stages(const Launch &L, cudaStream_t s)
 {
     auto kern = k_dense<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
-    const int ring = STAGES * stage_slots<CARRY>() * kThreads * (items_of<CARRY>() / 4) * (int)sizeof(int4);
+    const int ring = STAGES * kSlots * kThreads * (kItems / 4) * (int)sizeof(int4);
     const int smem = ring + (L.bitmap_ht ? (int)(((L.bitmap_len + 31) / 32) * 4) : 0);
     static const bool attr = [&] {  // once per instantiation, thread-safe
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring + (int)(kBitmapMax / 8));
@@ -2034,7 +2237,7 @@ int launch_stages(const Launch &L, cudaStream_t s)
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    const uint64_t tile = (uint64_t)kThreads * items_of<CARRY>();
+    const uint64_t tile = (uint64_t)kThreads * kItems;
     uint64_t blocks = (L.n + tile - 1) / tile;
     const uint64_t cap = (uint64_t)num_sms() * per_sm;
     if (blocks > cap) blocks = cap;
@@ -2046,24 +2249,15 @@ int launch_stages(const Launch &L, cudaStream_t s)
 }
 
 // Ring stages 3 or 2; rows carried between tiles (carry 1; 2: and the second
-// compaction level) only with compaction and a 2-stage ring; carry 3 (as 2,
-// and late slots) with a 2-stage ring of two slots and 8-row tiles per thread,
-// for a launch that prepare_late accepted.
+// compaction level) only with compaction and a 2-stage ring.
 template <class B, int TERM, int NREGS, int SPLIT, int... KS>
 int launch(const Launch &L, int stages, int carry, cudaStream_t s)
 {
     constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
-    constexpr bool kLate = kCompact && use_level2<SPLIT, KS...>(3);
-    if constexpr (B::bound || SPLIT == 0) {  // bound and SPLIT-0 passes are carry-3 passes
-        static_assert(kLate, "a bound shape needs the second level");
-        return launch_stages<B, TERM, NREGS, 2, SPLIT, 3, KS...>(L, s);
-    } else {
-        if (kLate && carry == 3) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kLate ? 3 : 0, KS...>(L, s);
-        if (stages >= 3) return launch_stages<Dyn, TERM, NREGS, 3, SPLIT, 0, KS...>(L, s);
-        if (kCompact && carry >= 2) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(L, s);
-        if (kCompact && carry == 1) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(L, s);
-        return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, 0, KS...>(L, s);
-    }
+    if (stages >= 3) return launch_stages<Dyn, TERM, NREGS, 3, SPLIT, 0, KS...>(L, s);
+    if (kCompact && carry >= 2) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(L, s);
+    if (kCompact && carry == 1) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(L, s);
+    return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, 0, KS...>(L, s);
 }
 
 // Slot bit of an operand (bit s: column slot s), and the slots an op reads.
@@ -2200,19 +2394,6 @@ bool convert(const ChainLaunch &C, int nregs, Launch &D)
     return true;
 }
 
-// Late slots of a chain whose ops from SPLIT on run on compacted rows with
-// the second level: the tail slots that neither the ops on 4-row groups nor
-// the first row-per-lane op read.  None when a row number does not fit 31
-// bits.
-template <int SPLIT>
-uint32_t late_slots_of(const Launch &D)
-{
-    if (D.n >= (1ull << 31)) return 0;
-    uint32_t early = 0;
-    for (int k = 0; k <= SPLIT && k < D.n_ops; k++) early |= op_slots(D.ops[k]);
-    return D.tail_slots & ~early;
-}
-
 // Whether the ops from index `split` on can run on compacted rows: no flags
 // output, and every later op only keeps or clears a row's flag (no NONE/OR
 // selection, no literal fill); ops before the split produce no register.
@@ -2276,13 +2457,11 @@ bool bound_ok(const Launch &D)
     return D.tail_slots == bound_tail<B, TERM, SPLIT, KS...>() && D.late_slots == late && late == (all & ~staged);
 }
 
-// Calls f.run<B, TERM, NREGS, SPLIT, KS...>() for the instantiation that
+// Calls f.run<Dyn, TERM, NREGS, SPLIT, KS...>() for the instantiation that
 // matches D, or returns SDB_ERR_UNSUPPORTED (without calling f).  `compact`:
-// 1 = compact after the first op when allowed; `bind`: a hot shape whose
-// operands match its canonical binding takes the bound pass (B), else B is
-// Dyn (only carry-3 launches, readied by prepare_late, bind).
+// 1 = compact after the first op when allowed.
 template <class F>
-int with_shape(const Launch &D, int term, int compact, F &f, bool bind = false)
+int with_shape(const Launch &D, int term, int compact, F &f)
 {
     int k[kMaxOps];
     for (int i = 0; i < D.n_ops; i++) k[i] = D.ops[i].kind;
@@ -2293,65 +2472,41 @@ int with_shape(const Launch &D, int term, int compact, F &f, bool bind = false)
     const bool r2 = D.nregs <= 2;
     // star join: semi + full + full -> group-by (SSB flight 2)
     if (r2 && term == T_GROUP && n == 3 && k[0] == SDB_OP_SEMI_PROBE && k[1] == SDB_OP_FULL_PROBE &&
-        k[2] == SDB_OP_FULL_PROBE) {
-        if (c1 && bind && bound_ok<StarBind, T_GROUP, 1, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>(D))
-            return f.template run<StarBind, T_GROUP, 2, 1, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>();
+        k[2] == SDB_OP_FULL_PROBE)
         return c1 ? f.template run<Dyn, T_GROUP, 2, 1, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>()
                   : f.template run<Dyn, T_GROUP, 2, 4, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>();
-    }
     // two semi probes -> flags (the flag-only front of a chain split in two)
     if (r2 && term == T_FLAGS && n == 2 && k[0] == SDB_OP_SEMI_PROBE && k[1] == SDB_OP_SEMI_PROBE)
         return f.template run<Dyn, T_FLAGS, 2, 3, SDB_OP_SEMI_PROBE, SDB_OP_SEMI_PROBE>();
-    // full + full + projection -> group-by (SSB flight 4 after its semi joins);
-    // under carry 3 (bind), with incoming flags, the rows are compacted on
-    // those flags before the first probe (SPLIT 0)
+    // full + full + projection -> group-by (SSB flight 4 after its semi joins)
     if (D.nregs <= 4 && term == T_GROUP && n == 3 && k[0] == SDB_OP_FULL_PROBE && k[1] == SDB_OP_FULL_PROBE &&
-        k[2] == SDB_OP_BINOP) {
-        if (bind && compact && D.flags_in && can_compact(D, term, 0)) {
-            if (bound_ok<Flight4Bind, T_GROUP, 0, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>(D))
-                return f.template run<Flight4Bind, T_GROUP, 4, 0, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>();
-            return f.template run<Dyn, T_GROUP, 4, 0, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>();
-        }
+        k[2] == SDB_OP_BINOP)
         return f.template run<Dyn, T_GROUP, 4, 4, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>();
-    }
     // full + full -> group-by
     if (r2 && term == T_GROUP && n == 2 && k[0] == SDB_OP_FULL_PROBE && k[1] == SDB_OP_FULL_PROBE)
         return f.template run<Dyn, T_GROUP, 2, 3, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>();
     // three full probes, the smallest table pre-tested by its bitmap
     // (prefilter_by_bitmap) -> three-key group-by (SSB flight 3)
     if (D.nregs <= 4 && term == T_GROUP && n == 4 && k[0] == SDB_OP_SEMI_PROBE && k[1] == SDB_OP_FULL_PROBE &&
-        k[2] == SDB_OP_FULL_PROBE && k[3] == SDB_OP_FULL_PROBE) {
-        if (c1 && bind &&
-            bound_ok<Flight3Bind, T_GROUP, 1, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>(D))
-            return f.template run<Flight3Bind, T_GROUP, 4, 1, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE,
-                                  SDB_OP_FULL_PROBE>();
+        k[2] == SDB_OP_FULL_PROBE && k[3] == SDB_OP_FULL_PROBE)
         return c1 ? f.template run<Dyn, T_GROUP, 4, 1, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE,
                                    SDB_OP_FULL_PROBE>()
                   : f.template run<Dyn, T_GROUP, 4, 5, SDB_OP_SEMI_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE,
                                    SDB_OP_FULL_PROBE>();
-    }
     // three full probes -> three-key group-by (none of the tables small enough for a bitmap)
     if (D.nregs <= 4 && term == T_GROUP && n == 3 && k[0] == SDB_OP_FULL_PROBE && k[1] == SDB_OP_FULL_PROBE &&
         k[2] == SDB_OP_FULL_PROBE)
         return f.template run<Dyn, T_GROUP, 4, 4, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE, SDB_OP_FULL_PROBE>();
     // range filter + one join + projection -> group-by
     if (r2 && term == T_GROUP && n == 3 && k[0] == SDB_OP_SEARCH_RANGE && k[1] == SDB_OP_FULL_PROBE &&
-        k[2] == SDB_OP_BINOP) {
-        if (c1 && bind && bound_ok<DateJoinBind, T_GROUP, 1, SDB_OP_SEARCH_RANGE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>(D))
-            return f.template run<DateJoinBind, T_GROUP, 2, 1, SDB_OP_SEARCH_RANGE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>();
+        k[2] == SDB_OP_BINOP)
         return c1 ? f.template run<Dyn, T_GROUP, 2, 1, SDB_OP_SEARCH_RANGE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>()
                   : f.template run<Dyn, T_GROUP, 2, 4, SDB_OP_SEARCH_RANGE, SDB_OP_FULL_PROBE, SDB_OP_BINOP>();
-    }
     // filter-project-sum (SSB flight 1)
     if (r2 && term == T_SUM && n == 4 && k[0] == SDB_OP_SEARCH_RANGE && k[1] == SDB_OP_SEARCH_RANGE &&
-        k[2] == SDB_OP_SELECT && k[3] == SDB_OP_BINOP) {
-        if (c1 && bind &&
-            bound_ok<FilterSumBind, T_SUM, 1, SDB_OP_SEARCH_RANGE, SDB_OP_SEARCH_RANGE, SDB_OP_SELECT, SDB_OP_BINOP>(D))
-            return f.template run<FilterSumBind, T_SUM, 2, 1, SDB_OP_SEARCH_RANGE, SDB_OP_SEARCH_RANGE, SDB_OP_SELECT,
-                                  SDB_OP_BINOP>();
+        k[2] == SDB_OP_SELECT && k[3] == SDB_OP_BINOP)
         return c1 ? f.template run<Dyn, T_SUM, 2, 1, SDB_OP_SEARCH_RANGE, SDB_OP_SEARCH_RANGE, SDB_OP_SELECT, SDB_OP_BINOP>()
                   : f.template run<Dyn, T_SUM, 2, 5, SDB_OP_SEARCH_RANGE, SDB_OP_SEARCH_RANGE, SDB_OP_SELECT, SDB_OP_BINOP>();
-    }
     if (r2 && term == T_SUM && n == 4 && k[0] == SDB_OP_SEARCH_RANGE && k[1] == SDB_OP_SEARCH_RANGE &&
         k[2] == SDB_OP_SEARCH_RANGE && k[3] == SDB_OP_BINOP)
         return c1 ? f.template run<Dyn, T_SUM, 2, 1, SDB_OP_SEARCH_RANGE, SDB_OP_SEARCH_RANGE, SDB_OP_SEARCH_RANGE,
@@ -2361,78 +2516,129 @@ int with_shape(const Launch &D, int term, int compact, F &f, bool bind = false)
     return SDB_ERR_UNSUPPORTED;
 }
 
+// The same for the late forms (D as to_late_form leaves it): SPLIT ops dense,
+// the rest on queued rows.  `bind`: operands that sit where the
+// shape's canonical binding puts them are read there (B), else B is Dyn.
+template <class F>
+int late_shape(const Launch &D, int term, F &f, bool bind = true)
+{
+    constexpr int R = SDB_OP_SEARCH_RANGE, S = SDB_OP_SELECT, SEMI = SDB_OP_SEMI_PROBE, FULL = SDB_OP_FULL_PROBE,
+                  BIN = SDB_OP_BINOP;
+    int k[kMaxOps] = {};
+    for (int i = 0; i < D.n_ops; i++) k[i] = D.ops[i].kind;
+    auto is = [&](int want_term, int nregs, std::initializer_list<int> kinds) {
+        return term == want_term && D.nregs <= nregs && D.n_ops == (int)kinds.size() && std::equal(kinds.begin(), kinds.end(), k);
+    };
+    if (is(T_GROUP, 2, {SEMI, K_HIT, FULL, FULL})) {
+        if (bind && bound_ok<StarBind, T_GROUP, 2, SEMI, K_HIT, FULL, FULL>(D))
+            return f.template run<StarBind, T_GROUP, 2, 2, SEMI, K_HIT, FULL, FULL>();
+        return f.template run<Dyn, T_GROUP, 2, 2, SEMI, K_HIT, FULL, FULL>();
+    }
+    if (is(T_GROUP, 2, {R, K_HIT, FULL, BIN})) {
+        if (bind && bound_ok<DateJoinBind, T_GROUP, 2, R, K_HIT, FULL, BIN>(D))
+            return f.template run<DateJoinBind, T_GROUP, 2, 2, R, K_HIT, FULL, BIN>();
+        return f.template run<Dyn, T_GROUP, 2, 2, R, K_HIT, FULL, BIN>();
+    }
+    if (is(T_GROUP, 4, {SEMI, K_HIT, FULL, FULL, FULL})) {
+        if (bind && bound_ok<Flight3Bind, T_GROUP, 2, SEMI, K_HIT, FULL, FULL, FULL>(D))
+            return f.template run<Flight3Bind, T_GROUP, 4, 2, SEMI, K_HIT, FULL, FULL, FULL>();
+        return f.template run<Dyn, T_GROUP, 4, 2, SEMI, K_HIT, FULL, FULL, FULL>();
+    }
+    if (D.flags_in && is(T_GROUP, 4, {K_HIT, FULL, FULL, BIN})) {
+        if (bind && bound_ok<Flight4Bind, T_GROUP, 1, K_HIT, FULL, FULL, BIN>(D))
+            return f.template run<Flight4Bind, T_GROUP, 4, 1, K_HIT, FULL, FULL, BIN>();
+        return f.template run<Dyn, T_GROUP, 4, 1, K_HIT, FULL, FULL, BIN>();
+    }
+    if (is(T_SUM, 2, {R, R, S, BIN})) {
+        if (bind && bound_ok<FilterSumBind, T_SUM, 2, R, R, S, BIN>(D))
+            return f.template run<FilterSumBind, T_SUM, 2, 2, R, R, S, BIN>();
+        return f.template run<Dyn, T_SUM, 2, 2, R, R, S, BIN>();
+    }
+    if (is(T_SUM, 2, {R, R, R, BIN})) return f.template run<Dyn, T_SUM, 2, 2, R, R, R, BIN>();
+    return SDB_ERR_UNSUPPORTED;
+}
+
+// Rewrites the ops of a chain whose rows can be carried into its late form:
+// the first probe that gives a value becomes a dense test of its table's hits
+// (K_HIT, eight rows of a thread probing together), and the probe itself runs
+// after the other probes, on the rows that are left, for its value.  The same
+// rows survive with the same registers.
+void to_late_form(Launch &D, int term)
+{
+    // with incoming flags the first op itself can be the probe
+    const int j = D.flags_in && D.ops[0].kind == SDB_OP_FULL_PROBE && can_compact(D, term, 0) ? 0 : 1;
+    if (D.n_ops <= j || D.n_ops >= kMaxOps || D.ops[j].kind != SDB_OP_FULL_PROBE || D.ops[j].a.src != 0) return;
+    Op ops[kMaxOps];
+    int n = 0;
+    for (int i = 0; i <= j; i++) ops[n++] = D.ops[i];
+    ops[j].kind = K_HIT;
+    int i = j + 1;
+    while (i < D.n_ops && D.ops[i].kind == SDB_OP_FULL_PROBE && D.ops[i].a.src == 0) ops[n++] = D.ops[i++];
+    ops[n++] = D.ops[j];
+    while (i < D.n_ops) ops[n++] = D.ops[i++];
+    for (int q = 0; q < n; q++) D.ops[q] = ops[q];
+    D.n_ops = n;
+}
+
+// Sets the tail and late slots of D's late form.
 struct LateProbe {
     Launch &D;
     template <class B, int TERM, int NREGS, int SPLIT, int... KS>
     int run()
     {
-        constexpr bool kLate = SPLIT <= (int)sizeof...(KS) && use_level2<SPLIT, KS...>(3);
-        if (SPLIT == 0 && kLate) D.tail_slots |= op_slots(D.ops[0]);  // rows compacted before the first op
-        D.late_slots = kLate ? late_slots_of<SPLIT>(D) : 0u;
+        uint32_t early = 0, tail = TERM != T_FLAGS ? slot_bit(D.value) : 0u;
+        for (int k = 0; k < D.n_ops; k++) (k < SPLIT ? early : tail) |= op_slots(D.ops[k]);
+        for (int q = 0; q < D.n_keys; q++) tail |= slot_bit(D.keys[q]);
+        D.tail_slots = tail;
+        D.late_slots = tail & ~early;
         return SDB_OK;
     }
 };
 
-// Fills D.late_slots for the instantiation with_shape picks with compaction.
-void set_late_slots(Launch &D, int term)
-{
-    LateProbe p{D};
-    if (with_shape(D, term, 1, p, true) != SDB_OK) D.late_slots = 0;
-}
-
-// Readies D for carry 3: finds its late slots and renumbers the slots so the
+// Readies D for its late pass: the late form, and the slots renumbered so the
 // staged ones come first (every operand, mask and pointer renamed alike).
-// False when the chain has no late slot or more than two staged ones; D then
-// stages every slot again (run_all_staged) and runs as it did under carry 2.
-void run_all_staged(Launch &D)
-{
-    D.late_slots = 0;
-    D.nstaged = D.nslot;
-}
-
+// False, D unchanged, when the chain has no late form, no late slot, more than
+// two staged ones, or row numbers that do not fit 31 bits.
 bool prepare_late(Launch &D, int term)
 {
-    set_late_slots(D, term);
-    if (!D.late_slots) {
-        run_all_staged(D);
-        return false;
-    }
+    if (D.n >= (1ull << 31)) return false;
+    Launch E = D;
+    to_late_form(E, term);
+    LateProbe p{E};
+    if (late_shape(E, term, p, false) != SDB_OK || !E.late_slots) return false;
     int perm[kSlots];
     int k = 0;
-    for (int s = 0; s < D.nslot; s++)
-        if (!((D.late_slots >> s) & 1u)) perm[s] = k++;
+    for (int s = 0; s < E.nslot; s++)
+        if (!((E.late_slots >> s) & 1u)) perm[s] = k++;
     const int staged = k;
-    for (int s = 0; s < D.nslot; s++)
-        if ((D.late_slots >> s) & 1u) perm[s] = k++;
+    if (staged > kLateSlots) return false;
+    for (int s = 0; s < E.nslot; s++)
+        if ((E.late_slots >> s) & 1u) perm[s] = k++;
     auto rename = [&](Src &x) {
         if (x.src == 0) x.idx = perm[x.idx];
     };
-    for (int i = 0; i < D.n_ops; i++) {
-        rename(D.ops[i].a);
-        rename(D.ops[i].b);
+    for (int i = 0; i < E.n_ops; i++) {
+        rename(E.ops[i].a);
+        rename(E.ops[i].b);
     }
-    rename(D.value);
-    for (int j = 0; j < D.n_keys; j++) rename(D.keys[j]);
+    rename(E.value);
+    for (int j = 0; j < E.n_keys; j++) rename(E.keys[j]);
     auto remask = [&](uint32_t m) {
         uint32_t r = 0;
-        for (int s = 0; s < D.nslot; s++)
+        for (int s = 0; s < E.nslot; s++)
             if ((m >> s) & 1u) r |= 1u << perm[s];
         return r;
     };
-    D.tail_slots = remask(D.tail_slots);
-    D.late_slots = remask(D.late_slots);
-    const int32_t *old[kSlots];
-    for (int s = 0; s < kSlots; s++) old[s] = D.slot[s];
-    for (int s = 0; s < D.nslot; s++) D.slot[perm[s]] = old[s];
-    D.nstaged = staged;
-    if (staged > stage_slots<3>()) {
-        run_all_staged(D);
-        return false;
-    }
+    E.tail_slots = remask(E.tail_slots);
+    E.late_slots = remask(E.late_slots);
+    for (int s = 0; s < E.nslot; s++) E.slot[perm[s]] = D.slot[s];
+    E.nstaged = staged;
+    D = E;
     return true;
 }
 
-// Shape identity of a launch: which kernel instantiation with_shape picks.
+// Shape identity of a launch: which kernel instantiation with_shape or
+// late_shape picks.
 struct ShapeProbe {
     int id = -1;
     template <class B, int TERM, int NREGS, int SPLIT, int... KS>
@@ -2446,6 +2652,39 @@ struct ShapeProbe {
     {
         static std::atomic<int> n{0};
         return n++;
+    }
+};
+
+// Blocks of a late pass's kernel for `want` units of work, with `words` words
+// of bitmap.
+template <class K>
+unsigned late_blocks(K kern, uint64_t want, uint32_t words)
+{
+    int per_sm = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, words * 4) != cudaSuccess || per_sm < 1)
+        per_sm = 1;
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)num_sms() * per_sm));
+}
+
+// Launches the late form's pass.
+struct LateLauncher {
+    const Launch &D;
+    cudaStream_t s;
+    template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+    int run()
+    {
+        auto kern = k_late<B, TERM, NREGS, SPLIT, KS...>;
+        static const bool attr = [&] {  // once per instantiation, thread-safe
+            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapMax / 8)) == cudaSuccess;
+        }();
+        (void)attr;
+        const uint32_t words = D.bitmap_ht ? (D.bitmap_len + 31) / 32 : 0;
+        constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
+        const unsigned blocks = late_blocks(kern, (D.n + kTile - 1) / kTile, words);
+        kern<<<blocks, kThreads, words * 4, s>>>(D);
+        g_dense_launches.fetch_add(1, std::memory_order_relaxed);
+        if (B::bound) g_bound_launches.fetch_add(1, std::memory_order_relaxed);
+        return sdb_check_launch("sdb_fused_chain (late)");
     }
 };
 
@@ -2469,9 +2708,13 @@ int dispatch(const ChainLaunch &C, int nregs, int term, int compact, int stages,
         carry = 2;  // as variant 7
         stages = 2;
     }
+    if (carry == 3) {
+        LateLauncher f{D, s};
+        return late_shape(D, term, f);
+    }
     if (!can_carry(D, term)) carry = 0;
     SingleLauncher f{D, stages, carry, s};
-    return with_shape(D, term, compact, f, carry == 3);
+    return with_shape(D, term, compact, f);
 }
 
 // One launch of k_batch over the chains of one shape group.
@@ -2480,7 +2723,7 @@ int batch_stages(const Launch *launches, const Span *spans, uint32_t n_spans, ui
                  cudaStream_t s)
 {
     auto kern = k_batch<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
-    const int ring = STAGES * stage_slots<CARRY>() * kThreads * (items_of<CARRY>() / 4) * (int)sizeof(int4);
+    const int ring = STAGES * kSlots * kThreads * (kItems / 4) * (int)sizeof(int4);
     const int smem = ring + (int)(bitmap_words * 4);
     static const bool attr = [&] {  // once per instantiation, thread-safe
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring + (int)(kBitmapMax / 8));
@@ -2512,30 +2755,42 @@ struct BatchLauncher {
     int run()
     {
         constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
-        constexpr bool kLate = kCompact && use_level2<SPLIT, KS...>(3);
-        if constexpr (B::bound || SPLIT == 0) {  // bound and SPLIT-0 passes are carry-3 passes
-            static_assert(kLate, "a bound shape needs the second level");
-            return batch_stages<B, TERM, NREGS, 2, SPLIT, 3, KS...>(launches, spans, n_spans, head, bitmap_words, s);
-        } else {
-            if (kLate && carry == 3)
-                return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kLate ? 3 : 0, KS...>(launches, spans, n_spans, head,
-                                                                                    bitmap_words, s);
-            if (stages >= 3)
-                return batch_stages<Dyn, TERM, NREGS, 3, SPLIT, 0, KS...>(launches, spans, n_spans, head,
-                                                                        bitmap_words, s);
-            if (kCompact && carry >= 2)
-                return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(launches, spans, n_spans,
-                                                                                       head, bitmap_words, s);
-            if (kCompact && carry == 1)
-                return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(launches, spans, n_spans,
-                                                                                       head, bitmap_words, s);
-            return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words,
-                                                                    s);
-        }
+        if (stages >= 3)
+            return batch_stages<Dyn, TERM, NREGS, 3, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words, s);
+        if (kCompact && carry >= 2)
+            return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(launches, spans, n_spans, head,
+                                                                                   bitmap_words, s);
+        if (kCompact && carry == 1)
+            return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(launches, spans, n_spans, head,
+                                                                                   bitmap_words, s);
+        return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words, s);
     }
 };
 
-// Whether with_shape binds D (its shape's bound pass runs it).
+struct LateBatchLauncher {
+    const Launch *launches;
+    const Span *spans;
+    uint32_t n_spans;
+    uint32_t *head;
+    uint32_t bitmap_words;
+    cudaStream_t s;
+    template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+    int run()
+    {
+        auto kern = k_batch_late<B, TERM, NREGS, SPLIT, KS...>;
+        static const bool attr = [&] {  // once per instantiation, thread-safe
+            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapMax / 8)) == cudaSuccess;
+        }();
+        (void)attr;
+        if (n_spans == 0) return SDB_OK;
+        kern<<<late_blocks(kern, n_spans, bitmap_words), kThreads, bitmap_words * 4, s>>>(launches, spans, n_spans, head);
+        g_dense_launches.fetch_add(1, std::memory_order_relaxed);
+        if (B::bound) g_bound_launches.fetch_add(1, std::memory_order_relaxed);
+        return sdb_check_launch("sdb_chain_batch_launch");
+    }
+};
+
+// Whether late_shape binds D (its shape's bound pass runs it).
 struct BoundProbe {
     bool bound = false;
     template <class B, int TERM, int NREGS, int SPLIT, int... KS>
@@ -2555,37 +2810,28 @@ constexpr bool has_pair_pass()
            std::is_same<B, FilterSumBind>::value;
 }
 
-template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
-int launch_pair_stages(LaunchPair &P, cudaStream_t s)
+template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+int launch_pair(LaunchPair &P, cudaStream_t s)
 {
-    auto kern = k_dense_pair<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
-    const int ring = STAGES * stage_slots<CARRY>() * kThreads * (items_of<CARRY>() / 4) * (int)sizeof(int4);
+    auto kern = k_late_pair<B, TERM, NREGS, SPLIT, KS...>;
     uint32_t words = 0;
     for (int c = 0; c < kPair; c++) {
         P.bits_off[c] = words;
         if (P.L[c].bitmap_ht) words += (P.L[c].bitmap_len + 31) / 32;
     }
-    const int smem = ring + (int)(words * 4);
     static const bool attr = [&] {  // once per instantiation, thread-safe
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring + kPair * (int)(kBitmapMax / 8));
-        return true;
+        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPair * (int)(kBitmapMax / 8)) == cudaSuccess;
     }();
     (void)attr;
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const uint64_t tile = (uint64_t)kThreads * items_of<CARRY>();
-    uint64_t blocks = (P.L[0].n + tile - 1) / tile;
-    const uint64_t cap = (uint64_t)num_sms() * per_sm;
-    if (blocks > cap) blocks = cap;
-    if (blocks == 0) blocks = 1;
-    kern<<<(unsigned)blocks, kThreads, smem, s>>>(P);
+    constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
+    const unsigned blocks = late_blocks(kern, (P.L[0].n + kTile - 1) / kTile, words);
+    kern<<<blocks, kThreads, words * 4, s>>>(P);
     g_dense_launches.fetch_add(1, std::memory_order_relaxed);
     g_bound_launches.fetch_add(1, std::memory_order_relaxed);
     return sdb_check_launch("sdb_chain_launch_pair");
 }
 
-// Whether the shape with_shape picks has a paired pass.
+// Whether the shape late_shape picks has a paired pass.
 struct PairProbe {
     bool ok = false;
     template <class B, int TERM, int NREGS, int SPLIT, int... KS>
@@ -2596,7 +2842,7 @@ struct PairProbe {
     }
 };
 
-// Launches the paired pass for the shape with_shape picks (bound, with a
+// Launches the paired pass for the shape late_shape picks (bound, with a
 // paired pass), else returns SDB_ERR_UNSUPPORTED without launching.
 struct PairLauncher {
     LaunchPair &P;
@@ -2605,13 +2851,13 @@ struct PairLauncher {
     int run()
     {
         if constexpr (B::bound && has_pair_pass<B>())
-            return launch_pair_stages<B, TERM, NREGS, 2, SPLIT, 3, KS...>(P, s);
+            return launch_pair<B, TERM, NREGS, SPLIT, KS...>(P, s);
         else
             return SDB_ERR_UNSUPPORTED;
     }
 };
 
-// Whether two launches readied for carry 3 (prepare_late) can share one
+// Whether two launches readied for their late pass (prepare_late) can share one
 // paired pass: the same bound shape, the same staged columns over the same
 // rows, no incoming or outgoing flags.
 bool pairable(const Launch &A, const Launch &B, int term_a, int term_b)
@@ -2622,10 +2868,10 @@ bool pairable(const Launch &A, const Launch &B, int term_a, int term_b)
     for (int i = 0; i < A.nstaged; i++)
         if (A.slot[i] != B.slot[i]) return false;
     ShapeProbe pa, pb;
-    if (with_shape(A, term_a, 1, pa, true) != SDB_OK || with_shape(B, term_b, 1, pb, true) != SDB_OK || pa.id != pb.id)
+    if (late_shape(A, term_a, pa) != SDB_OK || late_shape(B, term_b, pb) != SDB_OK || pa.id != pb.id)
         return false;
     PairProbe pp;
-    return with_shape(A, term_a, 1, pp, true) == SDB_OK && pp.ok;
+    return late_shape(A, term_a, pp) == SDB_OK && pp.ok;
 }
 
 }  // namespace dense
@@ -2719,7 +2965,7 @@ constexpr int kDenseVariant = 3;
 constexpr int kCompact2Variant = 5;  // as 4 with a 2-stage copy ring
 constexpr int kCarryVariant = 6;     // as 5, compacted rows carried across tiles
 constexpr int kLevel2Variant = 7;    // as 6, plus a second compaction after the first row-per-lane op
-constexpr int kLateVariant = 8;      // as 7, the columns read only after the second compaction loaded per row
+constexpr int kLateVariant = 8;      // the late passes
 constexpr int kMaxVariant = 8;
 
 int variant_stages(int v) { return (v == kCompact2Variant || v >= kCarryVariant) ? 2 : 3; }
@@ -3045,17 +3291,26 @@ int plan_batch(const sdb_chain_desc *chains, int n_chains, BatchPlan &bp)
         for (const Item &it : of[g]->items) {
             if (G.carry && !dense::can_carry(it.D, G.term)) G.carry = 0;  // every chain of the launch must allow it
             G.launches.push_back(it.D);
-            if (G.carry == 3 && !dense::prepare_late(G.launches.back(), G.term)) {
-                G.carry = 2;  // as variant 7
-                G.stages = 2;
-            }
             if (it.D.bitmap_ht) G.bitmap_words = std::max<uint32_t>(G.bitmap_words, (it.D.bitmap_len + 31) / 32);
         }
-        if (G.carry != 3)  // chains readied for carry 3 before the group fell back
-            for (dense::Launch &x : G.launches) dense::run_all_staged(x);
-        // spans in the launch's tiles (carry 3: 8 rows per thread, spans of half
+        if (G.carry == 3) {  // every chain in its late form, all of one shape, or none
+            std::vector<dense::Launch> late = G.launches;
+            int shape = -1;
+            for (dense::Launch &x : late) {
+                dense::ShapeProbe p;
+                if (!dense::prepare_late(x, G.term) || dense::late_shape(x, G.term, p, false) != SDB_OK ||
+                    (shape >= 0 && p.id != shape)) {
+                    G.carry = 2;  // as variant 7
+                    G.stages = 2;
+                    break;
+                }
+                shape = p.id;
+            }
+            if (G.carry == 3) G.launches.swap(late);
+        }
+        // spans in the launch's tiles (late passes: 8 rows per thread, spans of half
         // as many tiles)
-        const uint64_t tile = (uint64_t)kThreads * (G.carry == 3 ? dense::items_of<3>() : dense::kItems);
+        const uint64_t tile = (uint64_t)kThreads * (G.carry == 3 ? dense::kLateItems : dense::kItems);
         const uint64_t span = G.carry == 3 ? std::max<uint64_t>(S / 2, 1) : S;
         for (uint32_t c = 0; c < (uint32_t)G.launches.size(); c++) {
             const uint64_t tiles = (G.launches[c].n + tile - 1) / tile;
@@ -3065,7 +3320,7 @@ int plan_batch(const sdb_chain_desc *chains, int n_chains, BatchPlan &bp)
         G.bound = G.carry == 3;
         for (const dense::Launch &x : G.launches) {
             dense::BoundProbe p;
-            if (G.bound && dense::with_shape(x, G.term, 1, p, true) == SDB_OK) G.bound = p.bound;
+            if (G.bound && dense::late_shape(x, G.term, p) == SDB_OK) G.bound = p.bound;
             else G.bound = false;
         }
     }
@@ -3200,7 +3455,8 @@ int sdb_chain_batch_launch_part(const sdb_chain_batch *b, int part, sdb_stream_t
     }
     for (const auto &G : b->groups) {
         dense::BatchLauncher f{G.launches, G.spans, G.n_spans, G.head, G.bitmap_words, G.stages, G.carry, s};
-        int st = dense::with_shape(G.first, G.term, G.compact, f, G.bound);
+        dense::LateBatchLauncher fl{G.launches, G.spans, G.n_spans, G.head, G.bitmap_words, s};
+        int st = G.carry == 3 ? dense::late_shape(G.first, G.term, fl, G.bound) : dense::with_shape(G.first, G.term, G.compact, f);
         if (st != SDB_OK) return st;
     }
     for (const auto &c : b->singles) {
@@ -3295,13 +3551,13 @@ int sdb_chain_specialised(const sdb_chain_desc *chain)
     if (dense::with_shape(D, term, 1, probe) != SDB_OK) return 0;
     if (dense::can_carry(D, term) && dense::prepare_late(D, term)) {
         dense::BoundProbe bp;
-        if (dense::with_shape(D, term, 1, bp, true) == SDB_OK && bp.bound) return 2;
+        if (dense::late_shape(D, term, bp) == SDB_OK && bp.bound) return 2;
     }
     return 1;
 }
 
 // The paired pass.  A chain takes part as the single-chain pass would run it
-// under its tuned variant: only a carry-3 launch (variant 8) of a bound
+// under its tuned variant: only a late pass (variant 8) of a bound
 // shape pairs, so each chain's results are those of its own launch.
 static bool pair_launch_of(const sdb_chain_desc *c, dense::Launch &D, int &term)
 {
@@ -3324,9 +3580,9 @@ int sdb_chain_pair_key(const sdb_chain_desc *c, uint64_t *key)
     int term = 0;
     if (!pair_launch_of(c, D, term)) return 0;
     dense::PairProbe pp;
-    if (dense::with_shape(D, term, 1, pp, true) != SDB_OK || !pp.ok) return 0;
+    if (dense::late_shape(D, term, pp) != SDB_OK || !pp.ok) return 0;
     dense::ShapeProbe sp;
-    dense::with_shape(D, term, 1, sp, true);
+    dense::late_shape(D, term, sp);
     // FNV-1a over what pairable compares
     uint64_t h = 1469598103934665603ull;
     auto mix = [&](uint64_t v) {
@@ -3362,7 +3618,7 @@ int sdb_chain_launch_pair(const sdb_chain_desc *a, const sdb_chain_desc *b, sdb_
     if (!pair_launch_of(a, P.L[0], ta) || !pair_launch_of(b, P.L[1], tb) || !dense::pairable(P.L[0], P.L[1], ta, tb))
         return sdb_set_error(SDB_ERR_UNSUPPORTED, "sdb_chain_launch_pair: the chains do not share a paired pass");
     dense::PairLauncher f{P, (cudaStream_t)stream};
-    return dense::with_shape(P.L[0], ta, 1, f, true);
+    return dense::late_shape(P.L[0], ta, f);
 }
 
 }  // extern "C"
