@@ -51,6 +51,7 @@ from . import capi, plans, ssb
 HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_TABLE = os.path.join(HERE, "tuning", "gb300.json")
 VARIANTS = (0, 1, 2, 3, 4, 5, 6, 7, 8)
+LATE = 8
 TERMINALS = {"flags": 0, "sum": 1, "groupby": 2}
 
 OP_SEARCH_RANGE, OP_SEMI_PROBE, OP_FULL_PROBE = 1, 3, 4  # SDB_OP_* kinds of a chain's first op
@@ -141,20 +142,23 @@ def _time_variant(eng, plan, variant: int, reps: int) -> float:
     return statistics.median(ms)
 
 
-def tune(sizes: Iterable[int] = (1 << 20, 1 << 22, 1 << 24, 1 << 26, 120_000_000), reps: int = 5,
+def tune(sizes: Iterable[int] = (1 << 16, 1 << 18, 1 << 20, 1 << 22, 1 << 24, 1 << 26, 120_000_000), reps: int = 5,
          variants=VARIANTS, shapes=SHAPES, sf_dims: float = 20, log=print) -> dict:
     """Times every variant of every benchmark shape at each fact size on the
-    current device and returns the tuning table."""
+    current device and returns the tuning table.  Facts of 2^20 rows and more
+    join dimensions of ``sf_dims`` (fact partitions of a large schema),
+    smaller ones those of their own scale."""
     import torch
 
     from .engine import Engine
 
-    dims = ssb.gen_dims(sf_dims)
     cols = sorted({c for s in shapes for c in s[4]})
     timings: Dict[tuple, Dict[int, float]] = {}
     per_shape = []
     for n in sizes:
-        fact = ssb.gen_lineorder_device(int(n), cols, sf_dims, salt=7)
+        sf = sf_dims if n >= 1 << 20 else n / 6e6
+        dims = ssb.gen_dims(sf)
+        fact = ssb.gen_lineorder_device(int(n), cols, sf, salt=7)
         torch.cuda.synchronize()
         with Engine(fuse=True, profile=True) as eng:
             eng.load_table("lineorder", fact)
@@ -175,6 +179,8 @@ def tune(sizes: Iterable[int] = (1 << 20, 1 << 22, 1 << 24, 1 << 26, 120_000_000
     entries = []
     for (term, nregs, first_op, b), acc in sorted(timings.items()):
         best = min(acc, key=acc.get)
+        if acc.get(LATE, float("inf")) <= 1.1 * acc[best]:
+            best = LATE  # a near tie: the variant whose chains a batch can pair
         entries.append({"terminal": term, "nregs": nregs, "first_op": first_op, "rows_bucket": b, "variant": best,
                         "ms_sum": {str(v): t for v, t in acc.items()}})
     return {"device": torch.cuda.get_device_name(), "created": time.strftime("%Y-%m-%d %H:%M:%S"),
@@ -269,7 +275,7 @@ def tune_ops(sizes: Iterable[int] = (1 << 20, 1 << 22, 1 << 24, 1 << 26), reps: 
 def main(argv: Optional[List[str]] = None) -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("--out", required=True)
-    ap.add_argument("--sizes", default="1048576,4194304,16777216,67108864,120000000")
+    ap.add_argument("--sizes", default="65536,262144,1048576,4194304,16777216,67108864,120000000")
     ap.add_argument("--reps", type=int, default=5)
     ap.add_argument("--ops-only", action="store_true",
                     help="tune only the operator kernels' launch shapes and merge them into an existing --out table")

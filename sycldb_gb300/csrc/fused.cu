@@ -1361,33 +1361,41 @@ __device__ __forceinline__ void stage_bitmap(const LaunchT &L, uint32_t *s_bits)
 {
     if (!L.bitmap_ht) return;
     const uint32_t words = (L.bitmap_len + 31) / 32;
-    if (L.bitmap_kv) {  // a key/value table: entry j's occupancy word x == 1
-        const int4 *q = reinterpret_cast<const int4 *>(L.bitmap_ht);  // two entries per int4
-        for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) {
-            uint32_t bits = 0;
-            const uint32_t e0 = w * 32;
-            if (e0 + 32 <= L.bitmap_len) {
+    constexpr int kAhead = 8;
+    if (L.bitmap_kv) {
+        // a key/value table: entry j's occupancy word x == 1.  A warp votes on 32
+        // neighbouring entries at a time, eight words' reads in flight (40,000
+        // entries, 320 KB: with a thread packing its own 32 entries every
+        // read of a warp touched 32 lines, and a block took 75 us to start)
+        const int2 *e = reinterpret_cast<const int2 *>(L.bitmap_ht);
+        const uint32_t lane = threadIdx.x & 31u;
+        for (uint32_t w0 = threadIdx.x >> 5; w0 < words; w0 += kAhead * kThreads / 32) {
+            int32_t x[kAhead];
 #pragma unroll
-                for (int j = 0; j < 16; j++) {
-                    const int4 v = __ldg(q + e0 / 2 + j);
-                    bits |= ((uint32_t)(v.x == 1) | ((uint32_t)(v.z == 1) << 1)) << (2 * j);
-                }
-            } else {
-                const int2 *e = reinterpret_cast<const int2 *>(L.bitmap_ht);
-                for (uint32_t j = 0; j < 32 && e0 + j < L.bitmap_len; j++) bits |= (uint32_t)(e[e0 + j].x == 1) << j;
+            for (int j = 0; j < kAhead; j++) {
+                const uint32_t i = (w0 + j * (kThreads / 32)) * 32 + lane;
+                x[j] = i < L.bitmap_len ? __ldg(&e[i].x) : 0;
             }
-            s_bits[w] = bits;
+#pragma unroll
+            for (int j = 0; j < kAhead; j++) {
+                const uint32_t w = w0 + j * (kThreads / 32);
+                const uint32_t bits = __ballot_sync(0xffffffffu, x[j] == 1);
+                if (lane == 0 && w < words) s_bits[w] = bits;
+            }
         }
         return;
     }
+    const bool vec = sdb::aligned(L.bitmap_ht, 16);
     for (uint32_t w = threadIdx.x; w < words; w += blockDim.x) {
         uint32_t bits = 0;
         const uint32_t e0 = w * 32;
-        if (e0 + 32 <= L.bitmap_len && sdb::aligned(L.bitmap_ht, 4)) {
-            const uint32_t *q = reinterpret_cast<const uint32_t *>(L.bitmap_ht + e0);
+        if (e0 + 32 <= L.bitmap_len && vec) {
+            const uint4 *q = reinterpret_cast<const uint4 *>(L.bitmap_ht + e0);
+            const uint4 a = __ldg(q), b = __ldg(q + 1);
+            const uint32_t v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int j = 0; j < 8; j++) {
-                const uint32_t x = __vcmpne4(__ldg(q + j), 0u);
+                const uint32_t x = __vcmpne4(v[j], 0u);
                 bits |= (((x >> 7) & 1u) | ((x >> 14) & 2u) | ((x >> 21) & 4u) | ((x >> 28) & 8u)) << (4 * j);
             }
         } else {
