@@ -344,7 +344,9 @@ struct GroupArgs {
 __device__ __forceinline__ int64_t row_slot(const GroupArgs &a, uint64_t r)
 {
     uint32_t h = 0;
-    for (int j = 0; j < a.g; j++) h += ((uint32_t)a.keys[j][r] - (uint32_t)a.mins[j]) * a.mults[j];
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        if (j < a.g) h += ((uint32_t)a.keys[j][r] - (uint32_t)a.mins[j]) * a.mults[j];
     return sdb::group_slot(h, a.P);
 }
 
@@ -365,12 +367,12 @@ __device__ __forceinline__ void claim_keys(const GroupArgs &a, int64_t h, uint64
 template <bool SMEM>
 __device__ __forceinline__ void group_row(const GroupArgs &a, uint64_t r, uint32_t *s_lo, uint32_t *s_occ)
 {
+    const int32_t v = a.val[r];  // on its way with the keys
     const int64_t h = row_slot(a, r);
     if (h < 0 || (uint64_t)h >= a.P) {
         atomicAdd(&g_errors, 1ull);
         return;
     }
-    const int32_t v = a.val[r];
     if (SMEM) {
         if (s_occ[h] == 0u && atomicExch(&s_occ[h], 1u) == 0u) claim_keys(a, h, r);
         const uint32_t old = atomicAdd(&s_lo[h], (uint32_t)v);
@@ -383,64 +385,70 @@ __device__ __forceinline__ void group_row(const GroupArgs &a, uint64_t r, uint32
 }
 
 // Grid-stride over 16-row groups: a thread reads its group's 16 flags with
-// one 16-byte load (VEC: the flags are 16-byte aligned); the warp then lists
-// its flagged rows in shared memory (a warp prefix sum of the lanes' counts)
-// and updates them one row per lane, so the key and value loads of up to 32
-// flagged rows are in flight together instead of one row after another.
-constexpr int kGroupList = 32 * 16;  // a warp's rows per iteration
+// one 16-byte load (VEC: the flags are 16-byte aligned), the next chunk's on
+// their way meanwhile.  The flagged rows are queued per warp and updated one per lane,
+// 32 at a time, so that a warp does not wait for the key and value loads of
+// the few rows of a chunk.  512 threads share a table: with P = 7000 two blocks
+// fit an SM whatever their size.  30 M rows, 0.8 % flagged: 64 us with 256
+// threads and every chunk's rows updated at once, 48 with 512, 44 now.
+constexpr int kGroupThreads = 512;
 
 template <bool SMEM, bool VEC>
-__global__ void __launch_bounds__(kThreads) k_groupby(const GroupArgs a)
+__global__ void __launch_bounds__(kGroupThreads) k_groupby(const GroupArgs a)
 {
-    extern __shared__ uint32_t s_lo[];  // P low words, P high words, P occupancy words, the lists
+    constexpr uint32_t kWarps = kGroupThreads / 32;
+    extern __shared__ uint32_t s_lo[];  // P low words, P high words, P occupancy words
+    __shared__ uint64_t s_queue[kWarps][64];
     uint32_t *s_occ = s_lo + (SMEM ? 2 * a.P : 0);
-    uint32_t *s_list = s_occ + (SMEM ? a.P : 0);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t *list = s_list + warp * kGroupList;
+    uint64_t *queue = s_queue[warp];
+    uint32_t queued = 0;  // rows in it (warp-uniform)
     if (SMEM) {
         for (uint64_t i = threadIdx.x; i < 3 * a.P; i += blockDim.x) s_lo[i] = 0;
         __syncthreads();
     }
     const uint64_t groups = (a.n + 15) / 16;
-    const uint64_t wstride = (uint64_t)gridDim.x * (kThreads / 32);
+    const uint64_t wstride = (uint64_t)gridDim.x * kWarps;
+    // the flags of the lane's group in chunk c, as they are
+    auto load = [&](uint64_t c) {
+        const uint64_t r0 = (c * 32 + lane) * 16;
+        return VEC && r0 + 16 <= a.n ? __ldcs(reinterpret_cast<const uint4 *>(a.flags + r0)) : make_uint4(0, 0, 0, 0);
+    };
     // warp-uniform walk over chunks of 32 groups (512 rows)
-    for (uint64_t c = (uint64_t)blockIdx.x * (kThreads / 32) + warp; c * 32 < groups; c += wstride) {
+    uint64_t c = (uint64_t)blockIdx.x * kWarps + warp;
+    uint4 next = load(c);
+    for (; c * 32 < groups; c += wstride) {
         const uint64_t gi = c * 32 + lane;
         const uint64_t r0 = gi * 16;
+        const uint4 q = next;
+        next = load(c + wstride);
         uint32_t m = 0;  // bit b: row r0 + b is flagged
         if (gi < groups) {
             if (VEC && r0 + 16 <= a.n) {
-                const uint4 q = __ldcs(reinterpret_cast<const uint4 *>(a.flags + r0));
-                const uint32_t w[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-                for (int j = 0; j < 4; j++)
-#pragma unroll
-                    for (int b = 0; b < 4; b++) m |= (uint32_t)(((w[j] >> (8 * b)) & 0xffu) != 0) << (4 * j + b);
+                m = nz_bits4(q.x) | (nz_bits4(q.y) << 4) | (nz_bits4(q.z) << 8) | (nz_bits4(q.w) << 12);
             } else {
                 for (int b = 0; b < 16 && r0 + b < a.n; b++) m |= (uint32_t)(a.flags[r0 + b] != 0) << b;
             }
         }
-        // this lane's rows go to list[pos .. pos + popc(m))
-        const uint32_t cnt = __popc(m);
-        uint32_t pos = cnt;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, pos, o);
-            if (lane >= (uint32_t)o) pos += y;
+        // queue them, one of each lane at a time
+        for (;;) {
+            const unsigned any = __ballot_sync(0xffffffffu, m != 0);
+            if (any == 0) break;
+            if (m) {
+                queue[queued + __popc(any & ((1u << lane) - 1u))] = r0 + (uint32_t)__ffs(m) - 1u;
+                m &= m - 1;
+            }
+            queued += __popc(any);
+            __syncwarp();
+            if (queued >= 32) {
+                queued -= 32;
+                const uint64_t r = queue[queued + lane];
+                __syncwarp();  // read before the queue grows again
+                group_row<SMEM>(a, r, s_lo, s_occ);
+            }
         }
-        const uint32_t total = __shfl_sync(0xffffffffu, pos, 31);
-        pos -= cnt;
-        if (total == 0) continue;
-        while (m) {
-            const int b = __ffs(m) - 1;
-            m &= m - 1;
-            list[pos++] = lane * 16 + (uint32_t)b;
-        }
-        __syncwarp();
-        const uint64_t base = c * 32 * 16;
-        for (uint32_t i = lane; i < total; i += 32) group_row<SMEM>(a, base + list[i], s_lo, s_occ);
-        __syncwarp();
     }
+    if (lane < queued) group_row<SMEM>(a, queue[lane], s_lo, s_occ);
     if (SMEM) {
         __syncthreads();
         for (uint64_t i = threadIdx.x; i < a.P; i += blockDim.x)
@@ -1090,32 +1098,31 @@ int sdb_groupby_sum(const int32_t *const *keys, const int32_t *mins, const int32
     a.g = g; a.val = val; a.flags = flags; a.n = n; a.P = P; a.out_sum = out_sum; a.occ = occ;
     if (n == 0) return SDB_OK;
     cudaStream_t s = (cudaStream_t)stream;
-    // the slot table (P <= 8192: 12 B per slot) and every warp's row list
-    const size_t list_bytes = (size_t)(kThreads / 32) * kGroupList * sizeof(uint32_t);
-    const size_t smem = (P <= 8192 ? (size_t)P * 3 * sizeof(uint32_t) : 0) + list_bytes;
+    // the slot table (P <= 8192: 12 B per slot)
+    const size_t smem = P <= 8192 ? (size_t)P * 3 * sizeof(uint32_t) : 0;
     const uint64_t groups = (n + 15) / 16;
     const bool vec = sdb::aligned(flags, 16);
     static const bool attr_set = [] {  // once, thread-safe
-        const int most = 8192 * 12 + (kThreads / 32) * kGroupList * 4;
+        const int most = 8192 * 12;
         cudaFuncSetAttribute(k_groupby<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         cudaFuncSetAttribute(k_groupby<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
         return true;
     }();
     (void)attr_set;
-    // a block per 32 x 8 groups, capped at the resident blocks
-    const uint64_t want = (groups + 32 * (kThreads / 32) - 1) / (32 * (kThreads / 32));
+    // a block per 32 x 16 groups, capped at the resident blocks
+    const uint64_t want = (groups + kGroupThreads - 1) / kGroupThreads;
     if (P <= 8192) {
         const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sdb::device_sms() * 2));
         if (vec)
-            k_groupby<true, true><<<blocks, kThreads, smem, s>>>(a);
+            k_groupby<true, true><<<blocks, kGroupThreads, smem, s>>>(a);
         else
-            k_groupby<true, false><<<blocks, kThreads, smem, s>>>(a);
+            k_groupby<true, false><<<blocks, kGroupThreads, smem, s>>>(a);
     } else {
-        const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sdb::device_sms() * 8));
+        const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sdb::device_sms() * 4));
         if (vec)
-            k_groupby<false, true><<<blocks, kThreads, smem, s>>>(a);
+            k_groupby<false, true><<<blocks, kGroupThreads, smem, s>>>(a);
         else
-            k_groupby<false, false><<<blocks, kThreads, smem, s>>>(a);
+            k_groupby<false, false><<<blocks, kGroupThreads, smem, s>>>(a);
     }
     return sdb_check_launch("sdb_groupby_sum");
 }
