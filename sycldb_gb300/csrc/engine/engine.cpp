@@ -56,6 +56,11 @@ int sdb_sort_gather_small(const void *const *keys, const int *key_types, const i
                           const uint32_t *count, uint64_t cap, int ncols, const void *const *src, const int *wide,
                           void *const *dst, uint32_t *count_out, cudaStream_t s);  // sort.cu
 
+int sdb_copy_rows(uint64_t n, int ncols, const void *const *src, const int *wide, void *const *dst, uint32_t *count,
+                  cudaStream_t s);  // kernels.cu
+bool sdb_build_is_plain(const sdb_chain_desc *c);                           // fused.cu
+int sdb_build_few(const sdb_chain_desc *chains, int n, cudaStream_t s);  // fused.cu
+
 namespace sdb {
 
 constexpr uint64_t kDefaultSegment = 1ull << 28;  // common.hpp:12
@@ -859,6 +864,30 @@ struct Engine {
     // words directly instead.
     std::map<const uint8_t *, std::pair<const uint32_t *, uint64_t>> from_occ;
 
+    // Build chains of a plan that is not recorded, waiting to go out in one
+    // launch (sdb_build_few) before the plan's next other device operation.
+    std::vector<sdb_chain_desc> builds;
+
+    void flush_builds()
+    {
+        if (builds.empty()) return;
+        std::vector<sdb_chain_desc> now;
+        now.swap(builds);
+        if (now.size() == 1) check(sdb_fused_chain(&now[0], (sdb_stream_t)stream));
+        else check(sdb_build_few(now.data(), (int)now.size(), stream));
+    }
+
+    // Whether a build can wait with the others: it has the plain form and
+    // writes a table of its own (segments of one build side stay in order);
+    // timed launches go out one by one.
+    bool build_can_wait(const sdb_chain_desc &c) const
+    {
+        if (prof.on || builds.size() >= 4 || !sdb_build_is_plain(&c)) return false;
+        for (const sdb_chain_desc &o : builds)
+            if (o.ht_out == c.ht_out) return false;
+        return true;
+    }
+
     // Every device operation of a plan goes through here: run now on the
     // engine's stream, or recorded for a batch.
     void dev(const char *name, std::function<int(cudaStream_t)> fn, const sdb_chain_desc *chain = nullptr)
@@ -873,6 +902,7 @@ struct Engine {
             (pr.after ? pr.post : (pr.builds ? pr.mid : pr.pre)).push_back(std::move(op));
             return;
         }
+        flush_builds();
         cudaEvent_t a = nullptr;
         prof.begin(stream, name, a);
         check(fn(stream));
@@ -949,6 +979,8 @@ struct Engine {
             // plan's later work waits for it
             rec->chains.push_back(c);
             pr->after = true;
+        } else if (!rec && build && build_can_wait(c)) {
+            builds.push_back(c);
         } else {
             dev(build ? "build_chain" : "fused_chain",
                 [c](cudaStream_t s) { return sdb_fused_chain(&c, (sdb_stream_t)s); },
@@ -1300,8 +1332,8 @@ public:
             execute_pending_kernels();
             nrows = 1;
             flags = E.mm.alloc<uint8_t>(1);
-            uint8_t *f = flags;
-            E.dev("fill_flags", [f](cudaStream_t s) { return sdb_fill_u8(f, 1, 1, (sdb_stream_t)s); });
+            E.all_true.insert(flags);  // filled when something reads it
+            E.unfilled[flags] = 1;
             flags_secondary = nullptr;
             Column &rc = materialized_columns.emplace_back();
             rc.is_aggregate_result = true;
@@ -1969,6 +2001,7 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
     E.all_true.clear();
     E.unfilled.clear();
     E.from_occ.clear();
+    E.builds.clear();  // of a plan that failed
 
     std::deque<TransientTable> tts;
     std::vector<int> output_table(plan.rels.size(), -1);
@@ -2097,6 +2130,12 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
         auto oc = E.from_occ.find(fl0);
         const bool occ = oc != E.from_occ.end();
         const void *flags = occ ? static_cast<const void *>(oc->second.first) : fl0;
+        if (!occ && E.all_true.count(fl0) && cols.size() <= 8 && cnt < (1ull << 32)) {  // every row: no flags to read
+            E.dev("compact_gather", [cnt, src, wide, dst, count](cudaStream_t st) {
+                return sdb_copy_rows(cnt, (int)src.size(), src.data(), wide.data(), dst.data(), count, st);
+            });
+            continue;
+        }
         if (!occ) E.ensure_filled(fl0);
         if (cnt <= 65536 && cols.size() <= 8) {  // one launch
             E.dev("compact_gather", [flags, occ, cnt, src, wide, dst, count](cudaStream_t st) {
@@ -2113,6 +2152,7 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
                                             scratch, st);
         });
     }
+    E.flush_builds();
     // A small ordered result (one segment): sorted and gathered into pinned
     // memory by a launch that reads the count on the device, so that the host
     // waits once; a larger one, known by its count, goes through sort_result.

@@ -359,8 +359,8 @@ __host__ __device__ constexpr int min_blocks_of(int ITEMS) { return ITEMS <= 4 ?
 // the table is known to be zero (ht_zeroed: a miss would write a zero over a
 // zero).  A key outside the table is counted as an error and skipped, as in
 // the standalone builds.
-template <int ITEMS>
-__device__ __forceinline__ void build_store(const sdb_chain_desc &d, uint32_t rows, uint32_t live,
+template <int ITEMS, class DescT>
+__device__ __forceinline__ void build_store(const DescT &d, uint32_t rows, uint32_t live,
                                             const int32_t (&key)[ITEMS], const int32_t (&val)[ITEMS])
 {
     const bool kv = d.terminal == SDB_TERM_BUILD_KV;
@@ -429,10 +429,10 @@ __device__ __forceinline__ void build_rows(const sdb_chain_desc &d, const Tile<N
 // valid row writes), or after the tests for the live rows only (ht_zeroed),
 // so that a warp without a live row stops there.  The chain's parameters are
 // read once, before the tiles.
-template <bool STREAM, int ITEMS, int NT>
-__device__ __forceinline__ void build_tiles(const ChainLaunch &L, uint32_t t, uint32_t t_end, uint32_t stride)
+template <bool STREAM, int ITEMS, int NT, class LaunchT>
+__device__ __forceinline__ void build_tiles(const LaunchT &L, uint32_t t, uint32_t t_end, uint32_t stride)
 {
-    const sdb_chain_desc &d = L.d;
+    const auto &d = L.d;
     auto ld = [](const int32_t *p) { return STREAM ? __ldcs(p) : __ldg(p); };
     const uint32_t n = (uint32_t)d.n;  // interval-test chains have fewer than 2^32 rows
     const bool kv = d.terminal == SDB_TERM_BUILD_KV;
@@ -509,8 +509,8 @@ __device__ __forceinline__ void build_tiles(const ChainLaunch &L, uint32_t t, ui
     }
 }
 
-template <bool STREAM, int ITEMS>
-__device__ __forceinline__ void build_tiles_any(const ChainLaunch &L, uint32_t t, uint32_t t_end, uint32_t stride)
+template <bool STREAM, int ITEMS, class LaunchT>
+__device__ __forceinline__ void build_tiles_any(const LaunchT &L, uint32_t t, uint32_t t_end, uint32_t stride)
 {
     switch (L.n_tests) {
     case 0: build_tiles<STREAM, ITEMS, 0>(L, t, t_end, stride); break;
@@ -655,6 +655,39 @@ int launch_build(const ChainLaunch &L, int nregs, cudaStream_t s)
     if (nregs <= 2) return launch_term<T_BUILD, 2, 4>(L, s);
     if (nregs <= 4) return launch_term<T_BUILD, 4, 4>(L, s);
     return launch_term<T_BUILD, 8, 4>(L, s);
+}
+
+// The builds of one plan in one launch (a plan outside a batch has its tables
+// handed over one by one, all before its fact chain): up to kFewBuilds chains in
+// interval-test form, their records in the launch's own parameters, chain
+// blockIdx.y.  Each build is a few microseconds of launch and memory latency
+// whatever its size; three of them, 4.7 + 5.0 + 6.9 us, take 5.2 together.
+constexpr int kFewBuilds = 4;
+
+struct BuildLaunch {
+    struct {  // the fields of sdb_chain_desc that a build in interval-test form uses
+        uint64_t n;
+        const uint8_t *flags_in;
+        int32_t terminal;
+        sdb_operand build_key, build_val;
+        void *ht_out;
+        int32_t ht_min, ht_len, ht_zeroed, ht_log2;
+    } d;
+    int32_t n_tests;
+    RangeTest tests[kRangeTests];
+};
+
+struct FewBuilds {
+    BuildLaunch b[kFewBuilds];
+};
+
+constexpr int kFewItems = 4;
+
+__global__ void __launch_bounds__(kThreads, 4) k_build_few(const __grid_constant__ FewBuilds P)
+{
+    const BuildLaunch &L = P.b[blockIdx.y];
+    constexpr uint64_t kTile = (uint64_t)kThreads * kFewItems;
+    build_tiles_any<true, kFewItems>(L, blockIdx.x, (uint32_t)((L.d.n + kTile - 1) / kTile), gridDim.x);
 }
 
 // The build chains of a batch in one persistent launch.  Tile t of the batch
@@ -3630,3 +3663,48 @@ int sdb_chain_launch_pair(const sdb_chain_desc *a, const sdb_chain_desc *b, sdb_
 }
 
 }  // extern "C"
+
+// Whether a build chain can go into sdb_build_few: its ops are selections of
+// columns against literals.
+bool sdb_build_is_plain(const sdb_chain_desc *c)
+{
+    ChainLaunch L;
+    int nregs = 1, term = 0;
+    return sdb_chain_prepare(c, &L, sizeof L, &nregs, &term) == SDB_OK && term == T_BUILD && L.n_tests >= 0 && L.d.n > 0 &&
+           !L.d.flags_out;
+}
+
+// Up to four such chains, none writing a table that another writes, in one
+// launch.
+int sdb_build_few(const sdb_chain_desc *chains, int n, cudaStream_t s)
+{
+    if (n < 1 || n > kFewBuilds) return sdb_set_error(SDB_ERR_INVALID, "sdb_build_few: 1..%d chains", kFewBuilds);
+    FewBuilds P;
+    std::memset(&P, 0, sizeof P);
+    uint64_t most = 0;
+    for (int i = 0; i < n; i++) {
+        ChainLaunch L;
+        int nregs = 1, term = 0;
+        const int st = sdb_chain_prepare(&chains[i], &L, sizeof L, &nregs, &term);
+        if (st != SDB_OK) return st;
+        if (term != T_BUILD || L.n_tests < 0) return sdb_set_error(SDB_ERR_INVALID, "sdb_build_few: not a plain build");
+        BuildLaunch &b = P.b[i];
+        b.d.n = L.d.n;
+        b.d.flags_in = L.d.flags_in;
+        b.d.terminal = L.d.terminal;
+        b.d.build_key = L.d.build_key;
+        b.d.build_val = L.d.build_val;
+        b.d.ht_out = L.d.ht_out;
+        b.d.ht_min = L.d.ht_min;
+        b.d.ht_len = L.d.ht_len;
+        b.d.ht_zeroed = L.d.ht_zeroed;
+        b.d.ht_log2 = L.d.ht_log2;
+        b.n_tests = L.n_tests;
+        for (int t = 0; t < kRangeTests; t++) b.tests[t] = L.tests[t];
+        most = std::max(most, L.d.n);
+    }
+    const uint64_t tiles = (most + kThreads * kFewItems - 1) / (kThreads * kFewItems);
+    const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)num_sms() * 4));
+    k_build_few<<<dim3(blocks, (unsigned)n), kThreads, 0, s>>>(P);
+    return sdb_check_launch("sdb_build_few");
+}

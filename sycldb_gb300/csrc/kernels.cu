@@ -1491,6 +1491,39 @@ int sdb_op_tune_get(int op_kernel, uint64_t rows, int *block, int *blocks_per_sm
 
 }  // extern "C"
 
+namespace {
+// Every row of a segment (a result no filter applies to, a scalar sum): what
+// the compaction gives for flags that are all true, without flags.
+__global__ void __launch_bounds__(kThreads) k_copy_rows(const __grid_constant__ Compact a)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * kThreads;
+    for (uint64_t i = blockIdx.x * (uint64_t)kThreads + threadIdx.x; i < a.n; i += stride)
+        for (int c = 0; c < a.ncols; c++) {
+            if (a.wide[c]) static_cast<uint64_t *>(a.dst[c])[i] = static_cast<const uint64_t *>(a.src[c])[i];
+            else static_cast<int32_t *>(a.dst[c])[i] = static_cast<const int32_t *>(a.src[c])[i];
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) *a.count = (uint32_t)a.n;
+}
+}  // namespace
+
+// All rows of a segment (fewer than 2^32) copied from up to 8 columns.
+int sdb_copy_rows(uint64_t n, int ncols, const void *const *src, const int *wide, void *const *dst, uint32_t *count,
+                  cudaStream_t s)
+{
+    if (ncols > kCompactCols) return sdb_set_error(SDB_ERR_INVALID, "sdb_copy_rows: at most %d columns", kCompactCols);
+    Compact a{};
+    a.n = n;
+    a.ncols = ncols;
+    a.count = count;
+    for (int c = 0; c < ncols; c++) {
+        a.src[c] = src[c];
+        a.dst[c] = dst[c];
+        a.wide[c] = wide[c];
+    }
+    k_copy_rows<<<sdb::grid_for(n, kThreads, 8), kThreads, 0, s>>>(a);
+    return sdb_check_launch("sdb_copy_rows");
+}
+
 // The flagged rows of a segment of any size (flags or occupancy words, 16-byte
 // aligned) gathered from any number of columns: what sdb_compact_row_ids and
 // one sdb_gather_* per column give together.  Scratch as for

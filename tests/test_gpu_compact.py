@@ -106,3 +106,29 @@ def test_ordered_results_around_the_counted_sort_limit(qty, seg):
             at = np.lexsort((p.columns[1], p.columns[0]))
             for x, y in zip(g.columns, p.columns):
                 assert np.array_equal(x, y[at])
+
+
+@pytest.mark.parametrize("seg", [0, 4096])
+@pytest.mark.parametrize("join_tables", [0, 2])
+def test_builds_in_one_launch_and_unfiltered_results(seg, join_tables):
+    """Ad-hoc plans whose tables are built together: one to four of them, build
+    sides of one and of several segments (a table's segments stay in order),
+    direct and open-addressing tables; and results of every row, without
+    flags."""
+    ds = datasets.dataset(0.2)
+    b = plans.PlanBuilder()
+    b.scan("part")
+    b.project([plans.col(4), plans.col(0)])
+    every = b.plan()
+    b = plans.PlanBuilder()
+    b.scan("lineorder")
+    b.project([plans.col(12)])
+    b.aggregate([], 0)
+    total = b.plan()
+    pls = [plans.plan_date_join(1994), plans.plan_star(1, 3), plans.plan_star(2, 7, 1993, 1995, 9),
+           plans.plan_customer_supplier_date(2), plans.plan_profit(1), every, total]
+    with Engine(arena_bytes=1 << 30, segment_rows=seg, join_tables=join_tables) as eng:
+        for name, cols in ds.items():
+            eng.load_table(name, cols)
+        for plan in pls:
+            assert eng.execute(plan).canonical() == datasets.oracle_run(ds, plan, seg or (1 << 28))
