@@ -676,14 +676,15 @@ struct ProbeFullOA {
 // column on top it was 65.
 constexpr int kCompactRowsPerThread = 16;
 constexpr int kCompactChunk = kThreads * kCompactRowsPerThread;  // rows per count that callers' scratch is sized for
-constexpr uint32_t kCompactRows = 4 * kCompactChunk;              // rows a block lists at a time
+constexpr uint32_t kCompactRows = 4 * kCompactChunk;              // most rows a block lists at a time
 constexpr uint32_t kCompactTiles = 4096;                          // most tiles of a launch
 constexpr int kCompactCols = 8;                                   // columns gathered by one launch
 
 struct Compact {
     const void *flags;  // uint8 flags, or uint32 occupancy words (flag = word != 0)
     uint64_t n;
-    uint32_t subs;      // a tile is `subs` times kCompactRows rows
+    uint32_t steps;     // 16-row steps of a thread per list: 4, or 1 (a quarter of kCompactRows)
+    uint32_t subs;      // a tile is `subs` lists
     uint32_t *counts;   // per tile
     int32_t *ids;       // NULL: not wanted
     uint32_t *count;
@@ -768,14 +769,14 @@ __device__ __forceinline__ void put_rows(const Compact &a, const uint16_t *list,
 template <typename F>
 __global__ void __launch_bounds__(kThreads) k_compact_count(const __grid_constant__ Compact a)
 {
-    const uint64_t t0 = (uint64_t)blockIdx.x * a.subs * kCompactRows;
+    const uint64_t list_rows = (uint64_t)a.steps * kCompactChunk, t0 = blockIdx.x * a.subs * list_rows;
     uint32_t c = 0;
     for (uint32_t s = 0; s < a.subs; s++) {
-        const uint64_t r0 = t0 + (uint64_t)s * kCompactRows + threadIdx.x * 16u;
+        const uint64_t r0 = t0 + s * list_rows + threadIdx.x * 16u;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
             const uint64_t r = r0 + (uint64_t)j * kCompactChunk;
-            if (r < a.n) c += __popc(mask16(static_cast<const F *>(a.flags), r, a.n));
+            if (j < (int)a.steps && r < a.n) c += __popc(mask16(static_cast<const F *>(a.flags), r, a.n));
         }
     }
     uint32_t total;
@@ -788,14 +789,15 @@ __global__ void __launch_bounds__(kThreads) k_compact_write(const __grid_constan
 {
     __shared__ uint16_t s_list[kCompactRows];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t t0 = (uint64_t)blockIdx.x * a.subs * kCompactRows;
-    // warp w lists rows [2048 w, 2048 w + 2048): four steps of 16 rows per lane
+    const uint64_t list_rows = (uint64_t)a.steps * kCompactChunk, t0 = blockIdx.x * a.subs * list_rows;
+    // warp w lists rows [512 steps w, 512 steps (w + 1)): steps of 16 rows per lane
+    const uint32_t first = warp * 512u * a.steps + lane * 16u;
     uint32_t m[4];
     auto load = [&](uint64_t r0) {
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const uint64_t r = r0 + warp * 2048u + j * 512u + lane * 16u;
-            m[j] = r < a.n ? mask16(static_cast<const F *>(a.flags), r, a.n) : 0;
+            const uint64_t r = r0 + first + j * 512u;
+            m[j] = j < (int)a.steps && r < a.n ? mask16(static_cast<const F *>(a.flags), r, a.n) : 0;
         }
     };
     load(t0);  // in flight with the counts
@@ -804,7 +806,7 @@ __global__ void __launch_bounds__(kThreads) k_compact_write(const __grid_constan
     for (uint32_t t = threadIdx.x; t < blockIdx.x; t += kThreads) before += a.counts[t];
     block_exclusive_scan<kThreads>(before, &pos);
     for (uint32_t s = 0; s < a.subs; s++) {
-        const uint64_t r0 = t0 + (uint64_t)s * kCompactRows;
+        const uint64_t r0 = t0 + s * list_rows;
         if (r0 >= a.n) break;  // block-uniform
         if (s) load(r0);
         // the steps' lane prefixes, two 16-bit counts a word (at most 512 each)
@@ -830,7 +832,7 @@ __global__ void __launch_bounds__(kThreads) k_compact_write(const __grid_constan
         for (int j = 0; j < 4; j++) {
             uint32_t q = at + lanes[j], f = m[j];
             while (f) {
-                s_list[q++] = (uint16_t)(warp * 2048u + j * 512u + lane * 16u + (uint32_t)__ffs(f) - 1u);
+                s_list[q++] = (uint16_t)(first + j * 512u + (uint32_t)__ffs(f) - 1u);
                 f &= f - 1;
             }
             at += sums[j];
@@ -949,7 +951,12 @@ namespace {
 // there from an earlier call over the same flags).
 void launch_compact(Compact &a, bool occ, bool count_first, cudaStream_t s)
 {
-    const uint64_t lists = (a.n + kCompactRows - 1) / kCompactRows;
+    // lists of 4096 rows up to 4 M rows, so that a middling segment has blocks
+    // enough (437,500 slots, 27 blocks of 16384: 14.1 us for the two
+    // launches, 107 of 4096: 9.6)
+    a.steps = a.n <= (1ull << 22) ? 1 : 4;
+    const uint64_t list_rows = (uint64_t)a.steps * kCompactChunk;
+    const uint64_t lists = (a.n + list_rows - 1) / list_rows;
     a.subs = (uint32_t)((lists + kCompactTiles - 1) / kCompactTiles);
     const unsigned tiles = (unsigned)((lists + a.subs - 1) / a.subs);
     if (occ) {

@@ -36,7 +36,7 @@ def test_one_launch_compaction(n, share, occ, pad):
         assert np.array_equal(host(b, p, ids.size, c.dtype), c[ids])
 
 
-@pytest.mark.parametrize("n", [16_383, 16_384, 16_385, 5_000_001, (1 << 26) + 17])
+@pytest.mark.parametrize("n", [4095, 4096, 4097, 16_385, 1 << 22, (1 << 22) + 1, 5_000_001, (1 << 26) + 17])
 def test_row_ids_over_tiles(n):
     import torch
 
