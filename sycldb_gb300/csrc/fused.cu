@@ -2327,6 +2327,8 @@ void prefilter_by_bitmap(Launch &D, int terminal)
     for (int i = 0; i < D.n_ops; i++) {
         const Op &o = D.ops[i];
         if (o.kind != SDB_OP_FULL_PROBE || o.out_col || o.a.src != 0) return;
+        for (int q = 0; q < i; q++)
+            if (D.ops[q].out_reg == o.out_reg) return;  // the order of the two decides the register
         const uint64_t len = (uint64_t)((int64_t)o.hi - (int64_t)o.lo + 1);
         if (len >= 1 && len <= kBitmapMax && sdb::aligned(o.ht, 16) && len < best) {
             best = len;
@@ -2609,11 +2611,14 @@ void to_late_form(Launch &D, int term)
     // with incoming flags the first op itself can be the probe
     const int j = D.flags_in && D.ops[0].kind == SDB_OP_FULL_PROBE && can_compact(D, term, 0) ? 0 : 1;
     if (D.n_ops <= j || D.n_ops >= kMaxOps || D.ops[j].kind != SDB_OP_FULL_PROBE || D.ops[j].a.src != 0) return;
+    int i = j + 1;
+    for (; i < D.n_ops && D.ops[i].kind == SDB_OP_FULL_PROBE && D.ops[i].a.src == 0; i++)
+        if (D.ops[i].out_reg == D.ops[j].out_reg) return;  // the later probe's value is the one that stays
     Op ops[kMaxOps];
     int n = 0;
-    for (int i = 0; i <= j; i++) ops[n++] = D.ops[i];
+    for (i = 0; i <= j; i++) ops[n++] = D.ops[i];
     ops[j].kind = K_HIT;
-    int i = j + 1;
+    i = j + 1;
     while (i < D.n_ops && D.ops[i].kind == SDB_OP_FULL_PROBE && D.ops[i].a.src == 0) ops[n++] = D.ops[i++];
     ops[n++] = D.ops[j];
     while (i < D.n_ops) ops[n++] = D.ops[i++];

@@ -761,7 +761,7 @@ size_t scratch_layout(uint64_t n, char *base, Scratch *s)
 
 extern "C" {
 
-size_t sdb_sort_scratch_bytes(uint64_t n) { return scratch_layout(n, nullptr, nullptr); }
+size_t sdb_sort_scratch_bytes(uint64_t n) { return n <= kSmallSort ? 256 : scratch_layout(n, nullptr, nullptr); }
 
 int sdb_sort_rows(const void *const *keys, const int *key_types, const int *descending, int nkeys, uint64_t n,
                   uint32_t *perm, void *scratch, size_t scratch_bytes, sdb_stream_t stream)
@@ -771,7 +771,7 @@ int sdb_sort_rows(const void *const *keys, const int *key_types, const int *desc
     if (n > (1ull << 31)) return sdb_set_error(SDB_ERR_INVALID, "sdb_sort_rows: at most 2^31 rows");
     if (n == 0) return SDB_OK;
     if (!perm || !sdb::aligned(perm, 4)) return sdb_set_error(SDB_ERR_INVALID, "sdb_sort_rows: perm NULL or misaligned");
-    const size_t need = scratch_layout(n, nullptr, nullptr);
+    const size_t need = sdb_sort_scratch_bytes(n);
     if (!scratch || scratch_bytes < need || !sdb::aligned(scratch, 256))
         return sdb_set_error(SDB_ERR_INVALID, "sdb_sort_rows: scratch of %zu bytes (256-byte aligned) needed", need);
     SortKeys K{};

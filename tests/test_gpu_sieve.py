@@ -160,3 +160,38 @@ def test_sieve_equals_the_general_pass(n):
         for w, g in zip(want, got):
             assert np.array_equal(w, g), [(c.d.ops[k].kind, c.d.ops[k].logic_op) for k in range(c.d.n_ops)]
         release()
+
+
+@pytest.mark.parametrize("shape", ["star", "flight3", "full2"])
+@pytest.mark.parametrize("variant", [4, 7, 8])
+def test_probes_that_share_a_register(shape, variant):
+    """Chains of the specialised shapes whose probes write one register: the
+    last one's value is the row's, whatever order a pass probes in."""
+    rng = np.random.default_rng(5)
+    n = 60_013
+    c = Chain.__new__(Chain)
+    d = c.d = capi.ChainDesc()
+    c.n = d.n = n
+    kinds = {"star": [SEMI, FULL, FULL], "flight3": [FULL, FULL, FULL], "full2": [FULL, FULL]}[shape]
+    for i, kind in enumerate(kinds):
+        length = (2500, 300, 900)[i]
+        col = dev(rng.integers(0, length, n).astype(np.int32))[1]
+        op = d.ops[i]
+        op.kind, op.lo, op.hi, op.logic_op = kind, 0, length - 1, AND
+        set_col(op.a, col)
+        live = rng.random(length) < 0.7
+        if kind == SEMI:
+            op.ht = dev(live.astype(np.uint8))[1]
+        else:
+            op.ht = dev(np.stack([live.astype(np.int32), rng.integers(0, 20, length).astype(np.int32)], 1).reshape(-1))[1]
+            op.out_reg = 0
+    d.n_ops = len(kinds)
+    d.terminal = capi.TERM_GROUPBY
+    set_col(d.value, dev(rng.integers(-1000, 1000, n).astype(np.int32))[1])
+    d.n_keys, d.P = 1, 20
+    set_reg(d.keys[0], 0)
+    d.key_min[0], d.key_max[0] = 0, 19
+    st0, want = c.run(0)
+    st1, got = c.run(variant)
+    assert st0 == st1 == capi.SDB_OK and all(np.array_equal(w, g) for w, g in zip(want, got))
+    release()
