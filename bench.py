@@ -85,10 +85,10 @@ def _plan_date_join():
 
 # name -> (plan builder, fact columns key, dominant kernel)
 PLANS = {
-    "star": (_plan_star, "star", "k_dense (fused chain: semi + full + full probe, warp compaction, group-by; the "
-                                 "tuned variant, at SF20 the bound pass with late columns)"),
-    "filter_sum": (_plan_filter_sum, "q1", "k_dense (fused chain: range + range + select + projection, sum)"),
-    "date_join": (_plan_date_join, "q2", "k_dense (fused chain: range + full probe + projection, group-by)"),
+    "star": (_plan_star, "star", "k_late (fused chain: semi + full + full probe, group-by; the tuned variant, at SF20 the "
+                                 "bound pass with late columns)"),
+    "filter_sum": (_plan_filter_sum, "q1", "k_late (fused chain: range + range + select + projection, sum)"),
+    "date_join": (_plan_date_join, "q2", "k_late (fused chain: range + full probe + projection, group-by)"),
 }
 PROFILE_SUMMARY = os.path.join(ROOT, "profiles", "fused_chain_star_sf20.txt")
 
@@ -656,7 +656,7 @@ def run_configs(args, rank, stream, peak, ref):
             "rows_per_s": n / (ms / 1e3), "ms_per_step": ms, "steps": args.steps, "groups": len(rows),
             "l2": "%d copies of the fact columns (%.0f MB), step i reads copy i mod %d: inputs not L2-resident "
                   "between steps" % (copies, copies * alg / 1e6, copies),
-            "roofline": {"kernel": "k_dense (fused chain)", "bound": "hbm", "achieved": ach, "peak": peak,
+            "roofline": {"kernel": "k_late (fused chain)", "bound": "hbm", "achieved": ach, "peak": peak,
                          "unit": "GB/s", "frac": (ach / peak) if ach else None, "launch_ms": per,
                          "launches": kn, "algorithmic_bytes_per_launch": alg,
                          "traffic": profile_traffic(CONFIG_PROFILES[name], "traffic_bytes_per_launch:"),

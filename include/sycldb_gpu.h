@@ -617,8 +617,8 @@ int sdb_engine_last_plan_ms(const sdb_engine *eng, double *ms);
  * chains into one sdb_chain_batch.  A run replays: the zeroed region is
  * cleared, the plans' work before their chains runs spread over up to 8
  * streams, then the chain batch (one persistent launch per chain shape), then
- * the plans' remaining work and the copies of their results at full capacity
- * into pinned host staging.  Unless SDB_BATCH_EAGER, the replay is captured
+ * the plans' remaining work, whose compactions write the rows that there are
+ * into pinned host memory.  Unless SDB_BATCH_EAGER, the replay is captured
  * once as a CUDA graph and each run is one graph launch.  The base tables the
  * plans read must stay loaded, unchanged, while the batch lives.  Runs of one
  * batch must not overlap; different batches and plain executes may alternate
