@@ -2310,6 +2310,13 @@ inline uint32_t op_slots(const Op &o)
     return slot_bit(o.a) | (uses_b ? slot_bit(o.b) : 0u);
 }
 
+inline bool reads_reg(const Op &o)
+{
+    if (o.kind == SDB_OP_FILL) return false;
+    const bool uses_b = o.kind == SDB_OP_SELECT || o.kind == SDB_OP_BINOP;
+    return o.a.src == 1 || (uses_b && o.b.src == 1);
+}
+
 // Chains of two or three full probes (a star join whose dimensions all give
 // values, e.g. SSB flight 3): the probe whose table is the smallest (at most
 // kBitmapMax entries, 16-byte aligned) is first tested against a
@@ -2626,12 +2633,16 @@ void to_late_form(Launch &D, int term)
     D.n_ops = n;
 }
 
-// Sets the tail and late slots of D's late form.
+// Sets the tail and late slots of D's late form.  Unsupported when a dense op
+// reads a register: the late passes hold the staged columns there alone (no
+// op writes a register before them, so such a chain reads one that is zero).
 struct LateProbe {
     Launch &D;
     template <class B, int TERM, int NREGS, int SPLIT, int... KS>
     int run()
     {
+        for (int k = 0; k < SPLIT; k++)
+            if (reads_reg(D.ops[k])) return SDB_ERR_UNSUPPORTED;
         uint32_t early = 0, tail = TERM != T_FLAGS ? slot_bit(D.value) : 0u;
         for (int k = 0; k < D.n_ops; k++) (k < SPLIT ? early : tail) |= op_slots(D.ops[k]);
         for (int q = 0; q < D.n_keys; q++) tail |= slot_bit(D.keys[q]);
@@ -2643,8 +2654,9 @@ struct LateProbe {
 
 // Readies D for its late pass: the late form, and the slots renumbered so the
 // staged ones come first (every operand, mask and pointer renamed alike).
-// False, D unchanged, when the chain has no late form, no late slot, more than
-// two staged ones, or row numbers that do not fit 31 bits.
+// False, D unchanged, when the chain has no late form, a dense op that reads a
+// register, no late slot, more than two staged ones, or row numbers that do
+// not fit 31 bits.
 bool prepare_late(Launch &D, int term)
 {
     if (D.n >= (1ull << 31)) return false;
