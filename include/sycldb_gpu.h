@@ -255,6 +255,10 @@ int sdb_compact_gather_occ(const uint32_t *occ, uint64_t n, int ncols, const voi
 size_t sdb_sort_scratch_bytes(uint64_t n);
 int sdb_sort_rows(const void *const *keys, const int *key_types, const int *descending, int nkeys, uint64_t n,
                   uint32_t *perm, void *scratch, size_t scratch_bytes, sdb_stream_t stream);
+/* The same with the number of polls after which a wait inside the sort gives
+ * up (sdb_sort_rows: 2^20, about a second). */
+int sdb_sort_rows_polls(const void *const *keys, const int *key_types, const int *descending, int nkeys, uint64_t n,
+                        uint32_t *perm, void *scratch, size_t scratch_bytes, uint32_t polls, sdb_stream_t stream);
 
 /* ------------------------------------------------------ fused operator chain */
 
@@ -604,6 +608,10 @@ int sdb_engine_kernel_stats(const sdb_engine *eng, int k, const char **name, uin
                             double *total_ms);
 /* Device milliseconds of the last execute (CUDA events around the plan). */
 int sdb_engine_last_plan_ms(const sdb_engine *eng, double *ms);
+/* Polls after which a wait inside an ORDER BY of this engine gives up (2^20 at
+ * first; see sdb_sort_rows_polls).  The execute whose wait ran out returns
+ * SDB_ERR_TIMEOUT and no rows. */
+int sdb_engine_set_sort_polls(sdb_engine *eng, uint32_t polls);
 
 /* ---------------------------------------------------------------- batches
  * Many plans prepared once and run together.  No counterpart in the

@@ -132,6 +132,8 @@ _SIGS = {
     "sdb_sort_scratch_bytes": (c_size_t, [c_uint64]),
     "sdb_sort_rows": (c_int, [POINTER(c_void_p), POINTER(c_int), POINTER(c_int), c_int, c_uint64, _P, _P, c_size_t,
                               _P]),
+    "sdb_sort_rows_polls": (c_int, [POINTER(c_void_p), POINTER(c_int), POINTER(c_int), c_int, c_uint64, _P, _P, c_size_t,
+                                    c_uint32, _P]),
     "sdb_fused_chain": (c_int, [POINTER(ChainDesc), _P]),
     "sdb_fused_chain_variant": (c_int, [POINTER(ChainDesc), c_int, _P]),
     "sdb_chain_tune_set": (c_int, [c_int, c_int, c_uint64, c_int]),
@@ -174,6 +176,7 @@ _SIGS = {
     "sdb_result_free": (None, [c_void_p]),
     "sdb_engine_kernel_stats": (c_int, [c_void_p, c_int, POINTER(c_char_p), POINTER(c_uint64), POINTER(c_double)]),
     "sdb_engine_last_plan_ms": (c_int, [c_void_p, POINTER(c_double)]),
+    "sdb_engine_set_sort_polls": (c_int, [c_void_p, c_uint32]),
     "sdb_engine_batch_prepare": (c_int, [c_void_p, POINTER(c_char_p), c_int, c_int, POINTER(c_void_p)]),
     "sdb_batch_run": (c_int, [c_void_p, POINTER(c_void_p)]),
     "sdb_batch_info": (c_int, [c_void_p, POINTER(BatchStats)]),

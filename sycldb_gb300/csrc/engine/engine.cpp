@@ -55,7 +55,7 @@ int sdb_compact_gather_large(const void *flags, bool occ, uint64_t n, int ncols,
 int sdb_sort_gather_small(const void *const *keys, const int *key_types, const int *descending, int nkeys,
                           const uint32_t *count, uint64_t cap, int ncols, const void *const *src, const int *wide,
                           void *const *dst, uint32_t *count_out, cudaStream_t s);  // sort.cu
-
+const uint32_t *sdb_sort_failed(uint64_t n, void *scratch);  // sort.cu
 int sdb_copy_rows(uint64_t n, int ncols, const void *const *src, const int *wide, void *const *dst, uint32_t *count,
                   cudaStream_t s);  // kernels.cu
 bool sdb_build_is_plain(const sdb_chain_desc *c);                           // fused.cu
@@ -845,6 +845,7 @@ struct Engine {
     // compaction itself (one wait, no copy), other results' counts alone.
     char *pinned = nullptr;
     MemoryManager pin;
+    uint32_t sort_polls = 1u << 20;  // of a wait inside an ORDER BY before the query fails
     std::map<std::string, std::unique_ptr<Table>> tables;
     // Tables being loaded from column files in the background: installed by
     // the first plan that scans them (activate).
@@ -2182,7 +2183,8 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
 
 // ORDER BY on the device: the result rows of all segments are laid end to
 // end, sorted by the collation keys (sdb_sort_rows, stable) and gathered in
-// that order; pr then describes one segment of `total` rows.
+// that order; pr then describes one segment of `total` rows.  A sort whose
+// bounded wait ran out (its order is the rows' own) fails the query.
 void sort_result(Engine &E, PendingResult &pr, std::vector<uint32_t> &counts, uint64_t total)
 {
     const size_t ncols = pr.types.size();
@@ -2213,9 +2215,14 @@ void sort_result(Engine &E, PendingResult &pr, std::vector<uint32_t> &counts, ui
     const size_t sb = sdb_sort_scratch_bytes(total);
     void *scratch = E.mm.alloc<uint8_t>(sb);
     E.dev("sort_rows", [&](cudaStream_t s) {
-        return sdb_sort_rows(keys.data(), types.data(), desc.data(), (int)keys.size(), total, perm, scratch, sb,
-                             (sdb_stream_t)s);
+        return sdb_sort_rows_polls(keys.data(), types.data(), desc.data(), (int)keys.size(), total, perm, scratch, sb,
+                                   E.sort_polls, (sdb_stream_t)s);
     });
+    // the counts have left the pinned memory: its first word takes the sort's state
+    uint32_t *gave_up = reinterpret_cast<uint32_t *>(E.pinned);
+    *gave_up = 0;
+    if (const uint32_t *word = sdb_sort_failed(total, scratch))
+        SDB_CUDA(cudaMemcpyAsync(gave_up, word, sizeof *word, cudaMemcpyDeviceToHost, st));
     uint32_t *count = E.mm.alloc<uint32_t>(1);
     const uint32_t t32 = (uint32_t)total;
     SDB_CUDA(cudaMemcpyAsync(count, &t32, sizeof t32, cudaMemcpyHostToDevice, st));
@@ -2236,6 +2243,7 @@ void sort_result(Engine &E, PendingResult &pr, std::vector<uint32_t> &counts, ui
         }
     }
     SDB_CUDA(cudaStreamSynchronize(st));  // t32 lives on this frame
+    if (*gave_up) throw Error(SDB_ERR_TIMEOUT, "ORDER BY: a wait between the blocks of a sort pass ran out");
     pr.segs.assign(1, one);
     counts.assign(1, (uint32_t)total);
 }
@@ -2967,6 +2975,13 @@ int sdb_engine_destroy(sdb_engine *eng)
     if (E.stats_host) cudaFreeHost(E.stats_host);
     if (E.own_stream) cudaStreamDestroy(E.stream);
     delete eng;
+    return SDB_OK;
+}
+
+int sdb_engine_set_sort_polls(sdb_engine *eng, uint32_t polls)
+{
+    if (!eng) return sdb_set_error(SDB_ERR_INVALID, "sdb_engine_set_sort_polls: engine is NULL");
+    eng->E.sort_polls = polls;
     return SDB_OK;
 }
 

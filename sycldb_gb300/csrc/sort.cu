@@ -464,13 +464,14 @@ __global__ void __launch_bounds__(256) k_sort_plan(SortState *st, int head, int 
 // rows of the digit, kInclusive | c = it and all tiles before it hold c.
 constexpr uint32_t kInclusive = 0x80000000u;
 constexpr int kLookWindow = 8;        // earlier tiles read at a time
-constexpr uint32_t kLookLimit = 1u << 20;  // polls before a look-back gives up
+constexpr uint32_t kLookLimit = 1u << 20;  // polls before a look-back gives up, unless the caller says
 
 struct PassArgs {
     const void *col;
     int32_t wide, hi, desc;
     int32_t pass;
     uint32_t n;
+    uint32_t polls;       // of a look-back before it gives up
     SortState *st;
     uint32_t *look[2];    // [tiles][256] each
     uint32_t *perm[2];    // perm[0]: the caller's array, where the last active pass writes
@@ -501,13 +502,14 @@ __device__ __forceinline__ void store_look(uint32_t *p, uint32_t v)
 }
 
 // Rows of digit threadIdx.x in the tiles before `tile`: adds published counts
-// backwards until one covers all earlier tiles.  *ok = false when the wait
-// ran out.
-__device__ __forceinline__ uint32_t look_back(const uint32_t *look, uint32_t tile, const uint32_t *failed, bool &ok)
+// backwards until one covers all earlier tiles.  ok = false when the wait
+// ran out (after `limit` polls, or another tile's did).
+__device__ __forceinline__ uint32_t look_back(const uint32_t *look, uint32_t tile, const uint32_t *failed, uint32_t limit,
+                                              bool &ok)
 {
     uint32_t before = 0, polls = 0;
     int64_t t = (int64_t)tile - 1;  // the latest tile not added yet
-    for (;;) {
+    while (limit) {
         uint32_t v[kLookWindow];
 #pragma unroll
         for (int q = 0; q < kLookWindow; q++)
@@ -528,11 +530,10 @@ __device__ __forceinline__ uint32_t look_back(const uint32_t *look, uint32_t til
             }
         }
         if (done) return before;
-        if (++polls >= kLookLimit || ((polls & 1023u) == 0 && load_look(failed))) {
-            ok = false;
-            return before;
-        }
+        if (++polls >= limit || ((polls & 1023u) == 0 && load_look(failed))) break;
     }
+    ok = false;
+    return before;
 }
 
 // Keeps in `peers` the lanes whose `bit` is zero or not as this lane's is.
@@ -621,7 +622,7 @@ __device__ __forceinline__ bool pass_tile(const PassArgs &a, const PassPlan &pla
     uint32_t before = 0;
     if (threadIdx.x < 256 && tile) {
         bool ok = true;
-        before = look_back(look, tile, &a.st->failed, ok);
+        before = look_back(look, tile, &a.st->failed, a.polls, ok);
         if (!ok) {
             store_look(&a.st->failed, 1u);
             *s_stop = 1;
@@ -792,6 +793,12 @@ size_t sdb_sort_scratch_bytes(uint64_t n) { return n <= kSmallSort ? 256 : scrat
 int sdb_sort_rows(const void *const *keys, const int *key_types, const int *descending, int nkeys, uint64_t n,
                   uint32_t *perm, void *scratch, size_t scratch_bytes, sdb_stream_t stream)
 {
+    return sdb_sort_rows_polls(keys, key_types, descending, nkeys, n, perm, scratch, scratch_bytes, kLookLimit, stream);
+}
+
+int sdb_sort_rows_polls(const void *const *keys, const int *key_types, const int *descending, int nkeys, uint64_t n,
+                        uint32_t *perm, void *scratch, size_t scratch_bytes, uint32_t polls, sdb_stream_t stream)
+{
     if (nkeys < 1 || nkeys > kMaxKeys || !keys || !key_types || !descending)
         return sdb_set_error(SDB_ERR_INVALID, "sdb_sort_rows: 1..16 keys with types and directions");
     if (n > (1ull << 31)) return sdb_set_error(SDB_ERR_INVALID, "sdb_sort_rows: at most 2^31 rows");
@@ -839,6 +846,7 @@ int sdb_sort_rows(const void *const *keys, const int *key_types, const int *desc
     const unsigned hist_blocks = sdb::grid_for((n + 3) / 4, kHistThreads, 8);
     PassArgs a{};
     a.n = n32;
+    a.polls = polls;
     a.st = sc.st;
     for (int q = 0; q < 2; q++) {
         a.look[q] = sc.look[q];
@@ -879,6 +887,16 @@ int sdb_sort_rows(const void *const *keys, const int *key_types, const int *desc
 }
 
 }  // extern "C"
+
+// The device word that is not zero when a wait of the sort of n rows on this
+// scratch ran out (its order is then 0..n-1); NULL: no such sort waits.
+const uint32_t *sdb_sort_failed(uint64_t n, void *scratch)
+{
+    if (n <= kSmallSort) return nullptr;
+    Scratch sc;
+    scratch_layout(n, static_cast<char *>(scratch), &sc);
+    return &sc.st->failed;
+}
 
 // The rows of a result (*count of them, on the device, at most cap to be
 // ordered; cap <= 4096, up to 8 columns) written to dst in the order of the
