@@ -11,6 +11,7 @@
 #include <cstdint>
 #include <cuda_runtime.h>
 
+#include "smem_limit.hpp"
 #include "sycldb_gpu.h"
 
 namespace sdb {

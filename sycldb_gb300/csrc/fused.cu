@@ -2270,11 +2270,8 @@ int launch_stages(const Launch &L, cudaStream_t s)
     auto kern = k_dense<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
     const int ring = STAGES * kSlots * kThreads * (kItems / 4) * (int)sizeof(int4);
     const int smem = ring + (L.bitmap_ht ? (int)(((L.bitmap_len + 31) / 32) * 4) : 0);
-    static const bool attr = [&] {  // once per instantiation, thread-safe
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring + (int)(kBitmapMax / 8));
-        return true;
-    }();
-    (void)attr;
+    static sdb::SmemLimit smem_limit;  // one per instantiation
+    smem_limit.allow(ring + (int)(kBitmapMax / 8), kern);  // (a launch it was refused for reports it)
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
@@ -2732,10 +2729,8 @@ struct LateLauncher {
     int run()
     {
         auto kern = k_late<B, TERM, NREGS, SPLIT, KS...>;
-        static const bool attr = [&] {  // once per instantiation, thread-safe
-            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapMax / 8)) == cudaSuccess;
-        }();
-        (void)attr;
+        static sdb::SmemLimit smem_limit;  // one per instantiation
+        smem_limit.allow((int)(kBitmapMax / 8), kern);  // (a launch it was refused for reports it)
         const uint32_t words = D.bitmap_ht ? (D.bitmap_len + 31) / 32 : 0;
         constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
         const unsigned blocks = late_blocks(kern, (D.n + kTile - 1) / kTile, words);
@@ -2783,11 +2778,8 @@ int batch_stages(const Launch *launches, const Span *spans, uint32_t n_spans, ui
     auto kern = k_batch<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
     const int ring = STAGES * kSlots * kThreads * (kItems / 4) * (int)sizeof(int4);
     const int smem = ring + (int)(bitmap_words * 4);
-    static const bool attr = [&] {  // once per instantiation, thread-safe
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring + (int)(kBitmapMax / 8));
-        return true;
-    }();
-    (void)attr;
+    static sdb::SmemLimit smem_limit;  // one per instantiation
+    smem_limit.allow(ring + (int)(kBitmapMax / 8), kern);  // (a launch it was refused for reports it)
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;
@@ -2836,10 +2828,8 @@ struct LateBatchLauncher {
     int run()
     {
         auto kern = k_batch_late<B, TERM, NREGS, SPLIT, KS...>;
-        static const bool attr = [&] {  // once per instantiation, thread-safe
-            return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBitmapMax / 8)) == cudaSuccess;
-        }();
-        (void)attr;
+        static sdb::SmemLimit smem_limit;  // one per instantiation
+        smem_limit.allow((int)(kBitmapMax / 8), kern);  // (a launch it was refused for reports it)
         if (n_spans == 0) return SDB_OK;
         kern<<<late_blocks(kern, n_spans, bitmap_words), kThreads, bitmap_words * 4, s>>>(launches, spans, n_spans, head);
         g_dense_launches.fetch_add(1, std::memory_order_relaxed);
@@ -2877,10 +2867,8 @@ int launch_pair(LaunchPair &P, cudaStream_t s)
         P.bits_off[c] = words;
         if (P.L[c].bitmap_ht) words += (P.L[c].bitmap_len + 31) / 32;
     }
-    static const bool attr = [&] {  // once per instantiation, thread-safe
-        return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kPair * (int)(kBitmapMax / 8)) == cudaSuccess;
-    }();
-    (void)attr;
+    static sdb::SmemLimit smem_limit;  // one per instantiation
+    smem_limit.allow(kPair * (int)(kBitmapMax / 8), kern);  // (a launch it was refused for reports it)
     constexpr uint64_t kTile = (uint64_t)kThreads * kLateItems;
     const unsigned blocks = late_blocks(kern, (P.L[0].n + kTile - 1) / kTile, words);
     kern<<<blocks, kThreads, words * 4, s>>>(P);

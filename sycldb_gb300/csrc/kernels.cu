@@ -1109,13 +1109,8 @@ int sdb_groupby_sum(const int32_t *const *keys, const int32_t *mins, const int32
     const size_t smem = P <= 8192 ? (size_t)P * 3 * sizeof(uint32_t) : 0;
     const uint64_t groups = (n + 15) / 16;
     const bool vec = sdb::aligned(flags, 16);
-    static const bool attr_set = [] {  // once, thread-safe
-        const int most = 8192 * 12;
-        cudaFuncSetAttribute(k_groupby<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        cudaFuncSetAttribute(k_groupby<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-        return true;
-    }();
-    (void)attr_set;
+    static sdb::SmemLimit smem_limit;
+    smem_limit.allow(8192 * 12, k_groupby<true, true>, k_groupby<true, false>);
     // a block per 32 x 16 groups, capped at the resident blocks
     const uint64_t want = (groups + kGroupThreads - 1) / kGroupThreads;
     if (P <= 8192) {

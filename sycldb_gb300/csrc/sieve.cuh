@@ -717,11 +717,8 @@ int launch(const Launch &D, cudaStream_t s)
     constexpr int ring = kStages * kStaged * kThreads * kQ * (int)sizeof(int4);
     const int queues = TERM == T_FLAGS ? 0 : kWarps * (D.first_reg >= 0 ? 128 : 64) * 4;
     const int smem = ring + queues + (D.bitmap_ht ? (int)((D.bitmap_len + 31) / 32 * 4) : 0);
-    static const bool attr = [&] {  // once per instantiation, thread-safe
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ring + kWarps * 128 * 4 + (int)(kBitmapMax / 8));
-        return true;
-    }();
-    (void)attr;
+    static sdb::SmemLimit smem_limit;  // one per instantiation
+    smem_limit.allow(ring + kWarps * 128 * 4 + (int)(kBitmapMax / 8), kern);  // (a launch it was refused for reports it)
     int per_sm = 0;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem) != cudaSuccess || per_sm < 1)
         per_sm = 1;

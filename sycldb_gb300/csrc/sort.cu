@@ -835,13 +835,9 @@ int sdb_sort_rows_polls(const void *const *keys, const int *key_types, const int
     if (cudaMemsetAsync(sc.st, 0, reinterpret_cast<char *>(sc.look[1]) - reinterpret_cast<char *>(sc.st), s) != cudaSuccess)
         return sdb_set_error(SDB_ERR_CUDA, "sdb_sort_rows: memset failed");
     constexpr int kPassSmem = (2 * kSortTile + kSortWarps * 256) * 4;
-    static const bool attr = [] {  // once, thread-safe
-        bool ok = true;
-        for (auto f : {&k_sort_pass<0>, &k_sort_pass<8>, &k_sort_pass<16>, &k_sort_pass<24>})
-            ok &= cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPassSmem) == cudaSuccess;
-        return ok;
-    }();
-    if (!attr) return sdb_set_error(SDB_ERR_CUDA, "sdb_sort_rows: shared memory size refused");
+    static sdb::SmemLimit smem_limit;
+    if (!smem_limit.allow(kPassSmem, k_sort_pass<0>, k_sort_pass<8>, k_sort_pass<16>, k_sort_pass<24>))
+        return sdb_set_error(SDB_ERR_CUDA, "sdb_sort_rows: shared memory size refused");
     const int passes = words * 4;
     const unsigned hist_blocks = sdb::grid_for((n + 3) / 4, kHistThreads, 8);
     PassArgs a{};
