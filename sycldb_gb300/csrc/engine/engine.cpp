@@ -2131,7 +2131,7 @@ PendingResult run_plan(Engine &E, const std::string &plan_text)
         auto oc = E.from_occ.find(fl0);
         const bool occ = oc != E.from_occ.end();
         const void *flags = occ ? static_cast<const void *>(oc->second.first) : fl0;
-        if (!occ && E.all_true.count(fl0) && cols.size() <= 8 && cnt < (1ull << 32)) {  // every row: no flags to read
+        if (!occ && E.all_true.count(fl0) && cols.size() <= 8) {  // every row: no flags to read
             E.dev("compact_gather", [cnt, src, wide, dst, count](cudaStream_t st) {
                 return sdb_copy_rows(cnt, (int)src.size(), src.data(), wide.data(), dst.data(), count, st);
             });

@@ -1506,13 +1506,16 @@ __global__ void __launch_bounds__(kThreads) k_copy_rows(const __grid_constant__ 
         }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.count = (uint32_t)a.n;
 }
+
+constexpr uint64_t kMaxResultSegment = 1ull << 31;  // as sdb_compact_row_ids: row numbers and counts fit their words
 }  // namespace
 
-// All rows of a segment (fewer than 2^32) copied from up to 8 columns.
+// All rows of a segment (at most 2^31) copied from up to 8 columns.
 int sdb_copy_rows(uint64_t n, int ncols, const void *const *src, const int *wide, void *const *dst, uint32_t *count,
                   cudaStream_t s)
 {
     if (ncols > kCompactCols) return sdb_set_error(SDB_ERR_INVALID, "sdb_copy_rows: at most %d columns", kCompactCols);
+    if (n > kMaxResultSegment) return sdb_set_error(SDB_ERR_INVALID, "sdb_copy_rows: a segment of more than 2^31 rows");
     Compact a{};
     a.n = n;
     a.ncols = ncols;
@@ -1526,14 +1529,16 @@ int sdb_copy_rows(uint64_t n, int ncols, const void *const *src, const int *wide
     return sdb_check_launch("sdb_copy_rows");
 }
 
-// The flagged rows of a segment of any size (flags or occupancy words, 16-byte
-// aligned) gathered from any number of columns: what sdb_compact_row_ids and
-// one sdb_gather_* per column give together.  Scratch as for
+// The flagged rows of a segment of 1 to 2^31 rows (flags or occupancy words,
+// 16-byte aligned) gathered from any number of columns: what sdb_compact_row_ids
+// and one sdb_gather_* per column give together.  Scratch as for
 // sdb_compact_row_ids.  For the executor's results above sdb_compact_gather's
 // limits.
 int sdb_compact_gather_large(const void *flags, bool occ, uint64_t n, int ncols, const void *const *src, const int *wide,
                              void *const *dst, uint32_t *count, void *scratch, cudaStream_t s)
 {
+    if (n == 0 || n > kMaxResultSegment)
+        return sdb_set_error(SDB_ERR_INVALID, "sdb_compact_gather_large: a segment of no rows or more than 2^31");
     Compact a{};
     a.flags = flags;
     a.n = n;
