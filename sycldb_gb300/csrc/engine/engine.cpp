@@ -2921,6 +2921,9 @@ int sdb_engine_create(const sdb_engine_config *cfg, sdb_engine **out)
             if (E.cfg.segment_rows % 256 != 0) throw sdb::Error(SDB_ERR_INVALID, "segment_rows must be a multiple of 256");
             E.seg = E.cfg.segment_rows;
         }
+        // every refusal before anything is allocated
+        if (E.cfg.plan_cache < 0) throw sdb::Error(SDB_ERR_INVALID, "plan_cache must be >= 0");
+        if (E.cfg.join_tables < 0 || E.cfg.join_tables > 2) throw sdb::Error(SDB_ERR_INVALID, "join_tables must be 0, 1 or 2");
         if (E.cfg.stream) {
             E.stream = (cudaStream_t)E.cfg.stream;
         } else {
@@ -2938,13 +2941,12 @@ int sdb_engine_create(const sdb_engine_config *cfg, sdb_engine **out)
         SDB_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&E.pinned), sdb::kPinnedResult, cudaHostAllocDefault));
         E.pin.init_external(E.pinned, sdb::kPinnedResult, E.pinned, 0);
         E.prof.on = E.cfg.profile != 0;
-        if (E.cfg.plan_cache < 0) throw sdb::Error(SDB_ERR_INVALID, "plan_cache must be >= 0");
-        if (E.cfg.join_tables < 0 || E.cfg.join_tables > 2) throw sdb::Error(SDB_ERR_INVALID, "join_tables must be 0, 1 or 2");
         SDB_CUDA(cudaEventCreate(&E.plan_a));
         SDB_CUDA(cudaEventCreate(&E.plan_b));
         SDB_CUDA(cudaStreamSynchronize(E.stream));
     });
     if (st == SDB_OK) *out = eng.release();
+    else sdb_engine_destroy(eng.release());  // gives back what there is
     return st;
 }
 
