@@ -356,14 +356,15 @@ __device__ __forceinline__ void claim_keys(const GroupArgs &a, int64_t h, uint64
         for (int j = 0; j < a.g; j++) a.out_keys[j][h] = a.keys[j][r];
 }
 
-// Shared-memory privatised slot sums; a block's first touch of a slot also
-// runs the global first-writer exchange; sums flush once per touched slot.  A
-// slot's 64-bit sum is a low and a high word (s_lo[h], s_lo[P + h]) added with
-// 32-bit atomics, the low word's carry taken from the value its add returns:
-// 64-bit shared atomics are compare-and-swap loops (28 cycles of an SM per
-// warp over 280 slots, 450 over two; 9 and 19 this way).
 // One flagged row's slot update (K8): the first writer of a slot stores its
 // keys, the value goes into the slot's sum.
+//
+// SMEM: the sums are private to the block, in shared memory.  A block's first touch of a
+// slot also runs the global first-writer exchange; sums flush once per touched
+// slot.  A slot's 64-bit sum is a low and a high word (s_lo[h], s_lo[P + h])
+// added with 32-bit atomics, the low word's carry taken from the value its add
+// returns: 64-bit shared atomics are compare-and-swap loops (28 cycles of an SM
+// per warp over 280 slots, 450 over two; 9 and 19 this way).
 template <bool SMEM>
 __device__ __forceinline__ void group_row(const GroupArgs &a, uint64_t r, uint32_t *s_lo, uint32_t *s_occ)
 {
@@ -384,78 +385,146 @@ __device__ __forceinline__ void group_row(const GroupArgs &a, uint64_t r, uint32
     }
 }
 
-// Grid-stride over 16-row groups: a thread reads its group's 16 flags with
-// one 16-byte load (VEC: the flags are 16-byte aligned), the next chunk's on
-// their way meanwhile.  The flagged rows are queued per warp and updated one per lane,
-// 32 at a time, so that a warp does not wait for the key and value loads of
-// the few rows of a chunk.  512 threads share a table: with P = 7000 two blocks
-// fit an SM whatever their size.  30 M rows, 0.8 % flagged: 64 us with 256
-// threads and every chunk's rows updated at once, 48 with 512, 44 now.
-constexpr int kGroupThreads = 512;
-
-template <bool SMEM, bool VEC>
-__global__ void __launch_bounds__(kGroupThreads) k_groupby(const GroupArgs a)
+// Clears a block's private table / adds it to the global sums.
+template <int THREADS>
+__device__ __forceinline__ void group_reset(const GroupArgs &a, uint32_t *s_lo)
 {
-    constexpr uint32_t kWarps = kGroupThreads / 32;
+    for (uint64_t i = threadIdx.x; i < 3 * a.P; i += THREADS) s_lo[i] = 0;
+    __syncthreads();
+}
+
+template <int THREADS>
+__device__ __forceinline__ void group_flush(const GroupArgs &a, const uint32_t *s_lo, const uint32_t *s_occ)
+{
+    __syncthreads();
+    for (uint64_t i = threadIdx.x; i < a.P; i += THREADS)
+        if (s_occ[i])
+            atomicAdd(reinterpret_cast<unsigned long long *>(&a.out_sum[i]),
+                      (unsigned long long)s_lo[i] | ((unsigned long long)s_lo[a.P + i] << 32));
+}
+
+// Flags of the lane's 16 rows r0 .. r0 + 15 as a mask: one 16-byte load
+// (already made: q) where VEC and all 16 exist.
+template <bool VEC>
+__device__ __forceinline__ uint32_t group_mask(const GroupArgs &a, uint64_t r0, const uint4 &q)
+{
+    if (VEC && r0 + 16 <= a.n) return nz_bits4(q.x) | (nz_bits4(q.y) << 4) | (nz_bits4(q.z) << 8) | (nz_bits4(q.w) << 12);
+    uint32_t m = 0;
+    for (int b = 0; b < 16 && r0 + b < a.n; b++) m |= (uint32_t)(a.flags[r0 + b] != 0) << b;
+    return m;
+}
+
+template <bool VEC>
+__device__ __forceinline__ uint4 group_flags(const GroupArgs &a, uint64_t r0)
+{
+    return VEC && r0 + 16 <= a.n ? __ldcs(reinterpret_cast<const uint4 *>(a.flags + r0)) : make_uint4(0, 0, 0, 0);
+}
+
+// Queues the first row of each lane's mask (of rows r0 .. r0 + 15; `any`: the
+// lanes that have one) and updates the queue's last 32 once there are as many:
+// fewer than 32 before and after.
+template <bool SMEM>
+__device__ __forceinline__ void group_queue(const GroupArgs &a, uint32_t &m, unsigned any, uint64_t r0, uint64_t *queue,
+                                            uint32_t &queued, uint32_t *s_lo, uint32_t *s_occ)
+{
+    const uint32_t lane = threadIdx.x & 31u;
+    if (m) {
+        queue[queued + __popc(any & ((1u << lane) - 1u))] = r0 + (uint32_t)__ffs(m) - 1u;
+        m &= m - 1;
+    }
+    queued += __popc(any);
+    __syncwarp();
+    if (queued >= 32) {
+        queued -= 32;
+        const uint64_t r = queue[queued + lane];
+        __syncwarp();  // read before the queue grows again
+        group_row<SMEM>(a, r, s_lo, s_occ);
+    }
+}
+
+// The two forms walk chunks of 512 rows a warp, 16 rows a lane.
+//
+// Listed: the warp lists a chunk's flagged rows in row order (a prefix sum of the
+// lanes' counts) and updates them one per lane, so that the loads of a step
+// fall into neighbouring sectors and the steps of a chunk do not wait for one
+// another; the rows of a chunk with at most one per lane are queued over
+// chunks instead.  For the slots past shared memory, where every update goes to
+// the global arrays, and for inputs whose 512-thread blocks would leave SMs
+// empty.
+//
+// Queued: every flagged row is queued over chunks and updated one per lane, 32 at a
+// time, so that a warp does not wait for the key and value loads of the few
+// rows of a chunk; the next chunk's flags are on their way meanwhile.  512 threads
+// share a table: with P = 7000 two blocks fit an SM whatever their size.
+//
+// Both bound by the latency of the row loads and, where most rows are flagged,
+// by the atomics.  us, listed / queued, all rows flagged and 1 in 250:
+//   30 M rows, P = 100,000    297 / 398 and 17 / 16
+//   30 M rows, P = 7000       476 / 252 and 25 / 19
+//   400 K rows, P = 7000       21 / 25 and 6.4 / 6.5
+template <bool SMEM, bool VEC>
+__global__ void __launch_bounds__(kThreads) k_groupby_listed(const GroupArgs a)
+{
+    constexpr uint32_t kWarps = kThreads / 32;
     extern __shared__ uint32_t s_lo[];  // P low words, P high words, P occupancy words
     __shared__ uint64_t s_queue[kWarps][64];
+    __shared__ uint16_t s_list[kWarps][512];
     uint32_t *s_occ = s_lo + (SMEM ? 2 * a.P : 0);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint64_t *queue = s_queue[warp];
-    uint32_t queued = 0;  // rows in it (warp-uniform)
-    if (SMEM) {
-        for (uint64_t i = threadIdx.x; i < 3 * a.P; i += blockDim.x) s_lo[i] = 0;
-        __syncthreads();
-    }
-    const uint64_t groups = (a.n + 15) / 16;
-    const uint64_t wstride = (uint64_t)gridDim.x * kWarps;
-    // the flags of the lane's group in chunk c, as they are
-    auto load = [&](uint64_t c) {
-        const uint64_t r0 = (c * 32 + lane) * 16;
-        return VEC && r0 + 16 <= a.n ? __ldcs(reinterpret_cast<const uint4 *>(a.flags + r0)) : make_uint4(0, 0, 0, 0);
-    };
-    // warp-uniform walk over chunks of 32 groups (512 rows)
-    uint64_t c = (uint64_t)blockIdx.x * kWarps + warp;
-    uint4 next = load(c);
-    for (; c * 32 < groups; c += wstride) {
-        const uint64_t gi = c * 32 + lane;
-        const uint64_t r0 = gi * 16;
-        const uint4 q = next;
-        next = load(c + wstride);
-        uint32_t m = 0;  // bit b: row r0 + b is flagged
-        if (gi < groups) {
-            if (VEC && r0 + 16 <= a.n) {
-                m = nz_bits4(q.x) | (nz_bits4(q.y) << 4) | (nz_bits4(q.z) << 8) | (nz_bits4(q.w) << 12);
-            } else {
-                for (int b = 0; b < 16 && r0 + b < a.n; b++) m |= (uint32_t)(a.flags[r0 + b] != 0) << b;
-            }
+    uint16_t *list = s_list[warp];
+    uint32_t queued = 0;  // rows in the queue (warp-uniform)
+    if (SMEM) group_reset<kThreads>(a, s_lo);
+    for (uint64_t c = (uint64_t)blockIdx.x * kWarps + warp; c * 512 < a.n; c += (uint64_t)gridDim.x * kWarps) {
+        const uint64_t base = c * 512, r0 = base + lane * 16;
+        uint32_t m = group_mask<VEC>(a, r0, group_flags<VEC>(a, r0));
+        const uint32_t cnt = __popc(m);
+        if (!__any_sync(0xffffffffu, cnt > 1)) {
+            group_queue<SMEM>(a, m, __ballot_sync(0xffffffffu, cnt), r0, queue, queued, s_lo, s_occ);
+            continue;
         }
-        // queue them, one of each lane at a time
-        for (;;) {
-            const unsigned any = __ballot_sync(0xffffffffu, m != 0);
-            if (any == 0) break;
-            if (m) {
-                queue[queued + __popc(any & ((1u << lane) - 1u))] = r0 + (uint32_t)__ffs(m) - 1u;
-                m &= m - 1;
-            }
-            queued += __popc(any);
-            __syncwarp();
-            if (queued >= 32) {
-                queued -= 32;
-                const uint64_t r = queue[queued + lane];
-                __syncwarp();  // read before the queue grows again
-                group_row<SMEM>(a, r, s_lo, s_occ);
-            }
+        uint32_t pos = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, pos, o);
+            if (lane >= (uint32_t)o) pos += y;
         }
+        const uint32_t total = __shfl_sync(0xffffffffu, pos, 31);
+        pos -= cnt;
+        for (; m; m &= m - 1) list[pos++] = (uint16_t)(lane * 16 + (uint32_t)__ffs(m) - 1u);
+        __syncwarp();
+        for (uint32_t i = lane; i < total; i += 32) group_row<SMEM>(a, base + list[i], s_lo, s_occ);
+        __syncwarp();
     }
     if (lane < queued) group_row<SMEM>(a, queue[lane], s_lo, s_occ);
-    if (SMEM) {
-        __syncthreads();
-        for (uint64_t i = threadIdx.x; i < a.P; i += blockDim.x)
-            if (s_occ[i])
-                atomicAdd(reinterpret_cast<unsigned long long *>(&a.out_sum[i]),
-                          (unsigned long long)s_lo[i] | ((unsigned long long)s_lo[a.P + i] << 32));
+    if (SMEM) group_flush<kThreads>(a, s_lo, s_occ);
+}
+
+constexpr int kGroupThreads = 512;
+
+template <bool VEC>
+__global__ void __launch_bounds__(kGroupThreads) k_groupby_queued(const GroupArgs a)
+{
+    constexpr uint32_t kWarps = kGroupThreads / 32;
+    extern __shared__ uint32_t s_lo[];  // as above
+    __shared__ uint64_t s_queue[kWarps][64];
+    uint32_t *s_occ = s_lo + 2 * a.P;
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint64_t *queue = s_queue[warp];
+    uint32_t queued = 0;
+    group_reset<kGroupThreads>(a, s_lo);
+    const uint64_t wstride = (uint64_t)gridDim.x * kWarps;
+    uint64_t c = (uint64_t)blockIdx.x * kWarps + warp;
+    uint4 next = group_flags<VEC>(a, c * 512 + lane * 16);
+    for (; c * 512 < a.n; c += wstride) {
+        const uint64_t r0 = c * 512 + lane * 16;
+        uint32_t m = group_mask<VEC>(a, r0, next);
+        next = group_flags<VEC>(a, r0 + wstride * 512);
+        while (const unsigned any = __ballot_sync(0xffffffffu, m != 0))
+            group_queue<true>(a, m, any, r0, queue, queued, s_lo, s_occ);
     }
+    if (lane < queued) group_row<true>(a, queue[lane], s_lo, s_occ);
+    group_flush<kGroupThreads>(a, s_lo, s_occ);
 }
 
 struct OccToFlags {
@@ -1107,24 +1176,21 @@ int sdb_groupby_sum(const int32_t *const *keys, const int32_t *mins, const int32
     cudaStream_t s = (cudaStream_t)stream;
     // the slot table (P <= 8192: 12 B per slot)
     const size_t smem = P <= 8192 ? (size_t)P * 3 * sizeof(uint32_t) : 0;
-    const uint64_t groups = (n + 15) / 16;
     const bool vec = sdb::aligned(flags, 16);
     static sdb::SmemLimit smem_limit;
-    smem_limit.allow(8192 * 12, k_groupby<true, true>, k_groupby<true, false>);
-    // a block per 32 x 16 groups, capped at the resident blocks
-    const uint64_t want = (groups + kGroupThreads - 1) / kGroupThreads;
-    if (P <= 8192) {
-        const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sdb::device_sms() * 2));
-        if (vec)
-            k_groupby<true, true><<<blocks, kGroupThreads, smem, s>>>(a);
-        else
-            k_groupby<true, false><<<blocks, kGroupThreads, smem, s>>>(a);
+    smem_limit.allow(8192 * 12, k_groupby_listed<true, true>, k_groupby_listed<true, false>, k_groupby_queued<true>,
+                     k_groupby_queued<false>);
+    const uint64_t sms = (uint64_t)sdb::device_sms();
+    const uint64_t chunks = (n + 511) / 512;  // one per warp at a time
+    auto blocks = [&](int threads, uint64_t per_sm) {
+        return (unsigned)std::min<uint64_t>((chunks * 32 + threads - 1) / threads, sms * per_sm);
+    };
+    if (P > 8192) {
+        (vec ? k_groupby_listed<false, true> : k_groupby_listed<false, false>)<<<blocks(kThreads, 8), kThreads, 0, s>>>(a);
+    } else if (chunks * 32 < sms * kGroupThreads) {
+        (vec ? k_groupby_listed<true, true> : k_groupby_listed<true, false>)<<<blocks(kThreads, 2), kThreads, smem, s>>>(a);
     } else {
-        const unsigned blocks = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sdb::device_sms() * 4));
-        if (vec)
-            k_groupby<false, true><<<blocks, kGroupThreads, smem, s>>>(a);
-        else
-            k_groupby<false, false><<<blocks, kGroupThreads, smem, s>>>(a);
+        (vec ? k_groupby_queued<true> : k_groupby_queued<false>)<<<blocks(kGroupThreads, 2), kGroupThreads, smem, s>>>(a);
     }
     return sdb_check_launch("sdb_groupby_sum");
 }
