@@ -142,7 +142,23 @@ def _time_variant(eng, plan, variant: int, reps: int) -> float:
     return statistics.median(ms)
 
 
-def tune(sizes: Iterable[int] = (1 << 16, 1 << 18, 1 << 20, 1 << 22, 1 << 24, 1 << 26, 120_000_000), reps: int = 5,
+def choose(ms: Dict[int, float], bucket: int) -> int:
+    """The variant for a table entry whose variants took ``ms``: the fastest,
+    and on a near tie from 2^19 rows on the late form.  The entries are
+    measured with one plan per shape, of which 1 to 4 % of the rows are left
+    after the dense ops; the late form is the one that loses least when a plan
+    leaves more.  Late pass against the best other variant, us, where 10 to 16
+    and 50 % are left: filter-sum 1.2 M rows 12.7 / 15.4 and 14.6 / 15.4, star
+    900 K 22 / 24 and 36 / 47, star 120 M 755 / 917 and 1753 / 2066.  Below 2^19
+    it is not: its tiles of 2048 rows leave SMs with one block each (star
+    300 K, 16 %: 18 / 14)."""
+    best = min(ms, key=ms.get)
+    if bucket >= 19 and ms.get(LATE, float("inf")) <= 1.1 * ms[best]:
+        return LATE
+    return best
+
+
+def tune(sizes: Iterable[int] = (1 << 16, 1 << 18, 1 << 19, 1 << 20, 1 << 22, 1 << 24, 1 << 26, 120_000_000), reps: int = 5,
          variants=VARIANTS, shapes=SHAPES, sf_dims: float = 20, log=print) -> dict:
     """Times every variant of every benchmark shape at each fact size on the
     current device and returns the tuning table.  Facts of 2^20 rows and more
@@ -178,11 +194,8 @@ def tune(sizes: Iterable[int] = (1 << 16, 1 << 18, 1 << 20, 1 << 22, 1 << 24, 1 
     capi.force_chain_variant(-1)
     entries = []
     for (term, nregs, first_op, b), acc in sorted(timings.items()):
-        best = min(acc, key=acc.get)
-        if acc.get(LATE, float("inf")) <= 1.1 * acc[best]:
-            best = LATE  # a near tie: the variant whose chains a batch can pair
-        entries.append({"terminal": term, "nregs": nregs, "first_op": first_op, "rows_bucket": b, "variant": best,
-                        "ms_sum": {str(v): t for v, t in acc.items()}})
+        entries.append({"terminal": term, "nregs": nregs, "first_op": first_op, "rows_bucket": b,
+                        "variant": choose(acc, b), "ms_sum": {str(v): t for v, t in acc.items()}})
     return {"device": torch.cuda.get_device_name(), "created": time.strftime("%Y-%m-%d %H:%M:%S"),
             "reps": reps, "sizes": [int(n) for n in sizes], "entries": entries, "measurements": per_shape}
 
@@ -275,7 +288,7 @@ def tune_ops(sizes: Iterable[int] = (1 << 20, 1 << 22, 1 << 24, 1 << 26), reps: 
 def main(argv: Optional[List[str]] = None) -> int:
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
     ap.add_argument("--out", required=True)
-    ap.add_argument("--sizes", default="65536,262144,1048576,4194304,16777216,67108864,120000000")
+    ap.add_argument("--sizes", default="65536,262144,524288,1048576,4194304,16777216,67108864,120000000")
     ap.add_argument("--reps", type=int, default=5)
     ap.add_argument("--ops-only", action="store_true",
                     help="tune only the operator kernels' launch shapes and merge them into an existing --out table")

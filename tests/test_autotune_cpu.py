@@ -100,3 +100,17 @@ def test_operator_launch_shapes_set_get_and_load():
     finally:
         _clear_op_shapes()
         autotune.load_default()
+
+
+def test_the_committed_table_follows_the_rule():
+    """Every entry of the committed table is what the rule gives for its own
+    timings: the fastest variant, and the late form on a near tie of the
+    larger sizes alone."""
+    assert autotune.choose({7: 10.0, 8: 10.4}, 18) == 7
+    assert autotune.choose({7: 10.0, 8: 10.0}, 16) == 7
+    assert autotune.choose({7: 10.0, 8: 10.4}, 19) == 8
+    assert autotune.choose({7: 10.0, 8: 11.4}, 24) == 7
+    with open(autotune.DEFAULT_TABLE) as f:
+        table = json.load(f)
+    for e in table["entries"]:
+        assert e["variant"] == autotune.choose({int(v): t for v, t in e["ms_sum"].items()}, e["rows_bucket"]), e
