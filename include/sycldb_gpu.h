@@ -376,7 +376,8 @@ int sdb_fused_chain(const sdb_chain_desc *chain, sdb_stream_t stream);
  * those rows alone (only the sectors holding such rows; chains under 2^31
  * rows, else as 7).  Shapes without a
  * specialised pass fall back to the general pass, or (chains whose flags only
- * shrink) to the sieve, the late form's run-time counterpart.  Default (and an unset
+ * shrink) to the sieve, the late form's run-time counterpart. sdb_fused_chain sends
+ * them there from the rows on at which the sieve is the faster one.  Default (and an unset
  * tuning entry): 5. */
 int sdb_fused_chain_variant(const sdb_chain_desc *chain, int variant, sdb_stream_t stream);
 /* Tuning table used by sdb_fused_chain: variant for chains with this
@@ -410,6 +411,9 @@ int sdb_op_tune_get(int op_kernel, uint64_t rows, int *block, int *blocks_per_sm
  * reads every operand at a place fixed at compile time.  Host counters;
  * either pointer may be NULL. */
 int sdb_fused_launch_counts(uint64_t *specialised, uint64_t *bound);
+/* Launches of the sieve since the library loaded: the pass of the chains
+ * without a shape-specialised one whose flags only shrink (a host counter). */
+uint64_t sdb_sieve_launches(void);
 /* Registers (1..8) a chain needs, or a negative status if it is invalid. */
 int sdb_chain_registers(const sdb_chain_desc *chain);
 /* 2 when the chain has a shape-specialised instantiation (variants 3-8) and

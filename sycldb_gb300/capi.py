@@ -145,6 +145,7 @@ _SIGS = {
     "sdb_chain_pairable": (c_int, [POINTER(ChainDesc), POINTER(ChainDesc)]),
     "sdb_chain_pair_key": (c_int, [POINTER(ChainDesc), POINTER(c_uint64)]),
     "sdb_chain_launch_pair": (c_int, [POINTER(ChainDesc), POINTER(ChainDesc), c_void_p]),
+    "sdb_sieve_launches": (c_uint64, []),
     "sdb_fused_launch_counts": (c_int, [POINTER(c_uint64), POINTER(c_uint64)]),
     "sdb_chain_batch_scratch_bytes": (c_size_t, [POINTER(ChainDesc), c_int]),
     "sdb_chain_batch_create": (c_int, [POINTER(ChainDesc), c_int, _P, c_size_t, _P, POINTER(c_void_p)]),

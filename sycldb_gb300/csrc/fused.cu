@@ -3190,7 +3190,8 @@ static int fused_chain_impl(const sdb_chain_desc *chain, int variant, sdb_stream
     if (L.d.n == 0) return SDB_OK;
     cudaStream_t s = (cudaStream_t)stream;
     if (term == T_BUILD) return launch_build(L, nregs, s);
-    if (variant < 0) {
+    const bool asked = variant >= 0;  // by the caller, for any size
+    if (!asked) {
         variant = tune_entry(term, nregs, op_class(L.d), L.d.n);
         if (variant < 0) variant = kCompact2Variant;  // shape-specialised pass when one exists
     }
@@ -3198,7 +3199,7 @@ static int fused_chain_impl(const sdb_chain_desc *chain, int variant, sdb_stream
         const int st2 = dense::dispatch(L, nregs, term, variant != kDenseVariant, variant_stages(variant),
                                         variant_carry(variant), s);
         if (st2 != SDB_ERR_UNSUPPORTED) return st2;
-        const int st3 = sieve::dispatch(L, nregs, term, s);
+        const int st3 = sieve::dispatch(L, nregs, term, asked, s);
         if (st3 != SDB_ERR_UNSUPPORTED) return st3;
         variant = default_variant(nregs);
     }
@@ -3548,6 +3549,8 @@ int sdb_chain_tune_set_op(int terminal, int nregs, int first_op, uint64_t rows, 
         if (first_op < 0 || c == first_op) tune_entry(terminal, nregs, c, rows) = variant;
     return SDB_OK;
 }
+
+uint64_t sdb_sieve_launches(void) { return sieve::g_launches.load(std::memory_order_relaxed); }
 
 int sdb_fused_launch_counts(uint64_t *specialised, uint64_t *bound)
 {

@@ -467,6 +467,49 @@ __global__ void __launch_bounds__(kThreads, TERM == T_FLAGS ? 6 : 5) k_sieve(con
 }
 
 // ---------------------------------------------------------------- host
+// Rows from which a chain goes to the sieve, by its tests and probes.
+// Below, the general pass: its threads hold 8 rows of a column each and
+// sum or group them as they are, where the sieve lists every surviving row and
+// takes 32 at a time through its levels -- less work when few survive, more
+// when most do, and a tile of 2048 rows a block, too few of them on a small
+// input.  us, general / sieve, where 1 in 100, a half and all rows pass each test:
+//   SUM, a test          400 K  2.7/4.1  2.8/5.1  2.7/6.0    10 M  16/20  17/32  17/45
+//   SUM, test and probe  1 M    7.8/8.3 (a half)             10 M  55/46 (a half), 48/30 (1 in 20)
+//   SUM, two probes      1 M    11/8.6 (a half)              40 M  250/134
+//   group-by, two probes 400 K  0.7 to 1 of the general pass; four 0.7 to 0.9
+//   group-by, a test     400 K  7.5/6.4  9.6/10  8.3/12      40 M  178/67  210/189  204/303
+//   flags, a test        1 M    3.0/3.1                      10 M  15/13
+// A group-by whose P lies between the two passes' shared-memory tables
+// overflows the sieve's (1000 groups, 10 M rows, half of them left: 112/180).
+// Probes that give values alone may well drop nothing (a join with an unfiltered
+// dimension; one of them, group-by, 40 M rows: 344/606).  A chain whose tests
+// and semi joins drop nothing either is slower here, by up to a half (sums: up
+// to twice).
+inline uint64_t rows_from(const sdb_chain_desc &c, int term)
+{
+    if (term == T_FLAGS) return 1ull << 21;
+    int tests = 0, semi = 0, full = 0;
+    for (int i = 0; i < c.n_ops; i++) {
+        const int k = c.ops[i].kind;
+        tests += k == SDB_OP_SELECT || k == SDB_OP_SEARCH_RANGE || k == SDB_OP_SEARCH_POINTS;
+        semi += k == SDB_OP_SEMI_PROBE;
+        full += k == SDB_OP_FULL_PROBE;
+    }
+    if (tests + semi == 0) return ~0ull;
+    if (semi + full >= 3) return 0;
+    const bool between = term == T_GROUP && c.P > kDenseCap && c.P <= kCap;
+    if (semi + full == 2) return term == T_GROUP && !between ? 1ull << 17 : 1ull << 20;
+    if (term == T_GROUP) return between ? ~0ull : 1ull << 20;
+    return tests && semi + full ? 1ull << 23 : ~0ull;
+}
+
+// Rows from which a bitmap of a table of so many bytes is packed: every block
+// reads the whole table for it (200,000 key/value entries: 48 us, 16 as keys;
+// 20,000: 6).  Without one its probe reads the table's entries: 10 M rows, half
+// of them left by a test, group-by: 86 / 61 us with / without a bitmap of
+// 200,000 entries, 47 / 59 of 20,000.
+inline uint64_t bitmap_rows_from(uint64_t table_bytes) { return 64 * table_bytes; }
+
 // Turns a checked chain into a sieve launch.  False: the chain is left to the
 // general pass (a flag can come back after an op that is not a plain test of
 // columns, a column is written, a register is written twice or read before it
@@ -632,6 +675,7 @@ inline bool convert(const ChainLaunch &C, int nregs, int term, Launch &D)
         if ((o.kind != K_SEMI && o.kind != K_FULL) || o.ht_log2 || o.a.src != S_COL) continue;
         const uint64_t len = o.kmin <= o.kmax ? (uint64_t)((int64_t)o.kmax - (int64_t)o.kmin + 1) : 0;
         if (len < 1 || len > kBitmapMax || len >= best || (o.kind == K_FULL && !sdb::aligned(o.ht, 16))) continue;
+        if (c.n < bitmap_rows_from(len * (o.kind == K_FULL ? 8 : 1))) continue;
         best = len;
         bit = (int)i;
     }
@@ -710,6 +754,8 @@ inline bool convert(const ChainLaunch &C, int nregs, int term, Launch &D)
     return true;
 }
 
+std::atomic<uint64_t> g_launches{0};  // read by sdb_sieve_launches
+
 template <int TERM, int NREGS>
 int launch(const Launch &D, cudaStream_t s)
 {
@@ -725,12 +771,15 @@ int launch(const Launch &D, cudaStream_t s)
     const uint64_t tile = (uint64_t)kThreads * kItems;
     const uint64_t blocks = std::min<uint64_t>((D.n + tile - 1) / tile, (uint64_t)num_sms() * per_sm);
     kern<<<(unsigned)blocks, kThreads, smem, s>>>(D);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
     return sdb_check_launch("sdb_fused_chain (sieve)");
 }
 
-// SDB_ERR_UNSUPPORTED (nothing launched) when the chain is left to the general pass.
-inline int dispatch(const ChainLaunch &C, int nregs, int term, cudaStream_t s)
+// SDB_ERR_UNSUPPORTED (nothing launched) when the chain is left to the general
+// pass: it is not the sieve's, or, unless `any_size`, the general pass is faster.
+inline int dispatch(const ChainLaunch &C, int nregs, int term, bool any_size, cudaStream_t s)
 {
+    if (!any_size && C.d.n < rows_from(C.d, term)) return SDB_ERR_UNSUPPORTED;
     Launch D;
     if (!convert(C, nregs, term, D)) return SDB_ERR_UNSUPPORTED;
     if (term == T_FLAGS) return launch<T_FLAGS, 1>(D, s);
