@@ -189,8 +189,9 @@ struct Head {
     int exact;  // no key is cut or left out
 };
 
-// Bits for n rows: enough that rows of evenly spread keys seldom tie (6 bits
-// more than row ids have), in whole digits.
+// Bits for n rows, in whole digits: enough that rows of evenly spread keys
+// seldom tie (6 bits more than row ids have) up to 2^26 rows.  Above, a head that does not
+// hold the whole keys ties too often (k_sort_plan): every digit is sorted.
 __host__ __device__ inline int head_width(uint32_t n) { return n <= (1u << 18) ? 24 : 32; }
 
 // Bits of the first k keys' ranges, at most `width`.
@@ -536,7 +537,11 @@ __device__ __forceinline__ uint32_t look_back(const uint32_t *look, uint32_t til
     return before;
 }
 
-// Keeps in `peers` the lanes whose `bit` is zero or not as this lane's is.
+// Keeps in `peers` the lanes whose `bit` is zero or not as this lane's is: one
+// bit of the ballot match of GPU multisplit (Ashkiani, Davidson, Meyer, Owens,
+// 2016).  In PTX, so that the vote's predicate also turns the mask around; the
+// same in C++ (peers &= bit ? m : ~m, or by a shifted-out mask) took 686 and 617
+// us for a sort of 16.8 M rows by an int32 and a uint64 key, this 588.
 __device__ __forceinline__ void keep_same_bit(unsigned &peers, uint32_t bit)
 {
     asm volatile(
@@ -662,7 +667,7 @@ __device__ __forceinline__ bool pass_tile(const PassArgs &a, const PassPlan &pla
 // in runs of equal digits.  A wait that runs out marks the sort failed and
 // the block leaves; k_sort_finish then writes the identity.
 //
-// 16.8 M pairs: 108 us a pass (2.5 TB/s of the 16 bytes a pair moves), from
+// 16.8 M pairs: 100 to 103 us a pass (2.6 TB/s of the 16 bytes a pair moves), from
 // 210 us for the count, the three scans and the scatter that it replaces.
 // Bound by shared memory (half its cycles) and issue: the ballots are a third
 // of 115 warp instructions per 32 pairs.  __match_any_sync in their place
