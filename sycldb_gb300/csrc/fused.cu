@@ -1541,18 +1541,18 @@ __device__ __forceinline__ VRow<NREGS> take_row(const VRow<NREGS> &R, const uint
 
 // The ops after the first row-per-lane op and the terminal, for the rows of
 // a level-2 group (lane j: row j while F.live).
-template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_run(const Launch &L, VRow<NREGS> &F, const uint32_t *s_bits, uint32_t *s_key,
                                            uint32_t *s_sum, bool direct, uint64_t &acc)
 {
     constexpr int N = sizeof...(KS);
-    run_steps1<B, NREGS, SPLIT + 1, KS...>(L, F, s_bits, std::make_integer_sequence<int, N - SPLIT - 1>{});
-    finish_row<TERM, B>(L, F, s_key, s_sum, direct, acc);
+    run_steps1<Dyn, NREGS, SPLIT + 1, KS...>(L, F, s_bits, std::make_integer_sequence<int, N - SPLIT - 1>{});
+    finish_row<TERM, Dyn>(L, F, s_key, s_sum, direct, acc);
 }
 
 // After the first row-per-lane op of a group: appends its live rows to the
 // level-2 rows and runs the remaining ops whenever 32 are pending.
-template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_push(const Launch &L, const VRow<NREGS> &R, Level2<NREGS> &Q,
                                             const uint32_t *s_bits, uint32_t *s_key, uint32_t *s_sum,
                                             bool direct, uint64_t &acc)
@@ -1574,7 +1574,7 @@ __device__ __forceinline__ void level2_push(const Launch &L, const VRow<NREGS> &
     if (n2 + cnt >= 32) {
         VRow<NREGS> F = Q.r;
         F.live = true;
-        level2_run<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, F, s_bits, s_key, s_sum, direct, acc);
+        level2_run<TERM, NREGS, SPLIT, CARRY, KS...>(L, F, s_bits, s_key, s_sum, direct, acc);
         const uint32_t used = 32 - n2;
         const VRow<NREGS> got = take_row(R, Q.src, lane + used, cnt);
         if (lane < cnt - used) Q.r = got;
@@ -1594,19 +1594,19 @@ __host__ __device__ constexpr bool use_level2(int carry)
 }
 
 // The first row-per-lane op and then the second level, for one group.
-template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void level2_group(const Launch &L, VRow<NREGS> &R, Level2<NREGS> &Q, const uint32_t *s_bits,
                                              uint32_t *s_key, uint32_t *s_sum, bool direct, uint64_t &acc)
 {
     constexpr int kinds[] = {KS...};
 #pragma unroll
     for (int i = 0; i < NREGS; i++) R.reg[i] = 0;
-    step1<kinds[SPLIT], B::a(SPLIT), B::b(SPLIT), B::out(SPLIT)>(L.ops[SPLIT], R, s_bits);
-    level2_push<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, R, Q, s_bits, s_key, s_sum, direct, acc);
+    step1<kinds[SPLIT], kAny, kAny, kAny>(L.ops[SPLIT], R, s_bits);
+    level2_push<TERM, NREGS, SPLIT, CARRY, KS...>(L, R, Q, s_bits, s_key, s_sum, direct, acc);
 }
 
 // Runs whatever the warp still holds (at the end of a block's rows of a chain).
-template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void drain_carry(const Launch &L, uint32_t &carry, const int4 &ce, Level2<NREGS> &Q,
                                             const uint32_t *s_bits, uint32_t *s_key, uint32_t *s_sum,
                                             bool direct, uint64_t &acc)
@@ -1621,16 +1621,16 @@ __device__ __forceinline__ void drain_carry(const Launch &L, uint32_t &carry, co
         R.v3 = e.w;
         R.live = lane < carry;
         if constexpr (use_level2<SPLIT, KS...>(CARRY))
-            level2_group<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, R, Q, s_bits, s_key, s_sum, direct, acc);
+            level2_group<TERM, NREGS, SPLIT, CARRY, KS...>(L, R, Q, s_bits, s_key, s_sum, direct, acc);
         else
-            sparse_row<TERM, B, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
+            sparse_row<TERM, Dyn, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
     }
     carry = 0;
     if constexpr (use_level2<SPLIT, KS...>(CARRY)) {
         if (Q.n) {
             VRow<NREGS> F = Q.r;
             F.live = lane < Q.n;
-            level2_run<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, F, s_bits, s_key, s_sum, direct, acc);
+            level2_run<TERM, NREGS, SPLIT, CARRY, KS...>(L, F, s_bits, s_key, s_sum, direct, acc);
         }
         Q.n = 0;
     }
@@ -1645,7 +1645,7 @@ __device__ __forceinline__ int32_t tail_value(const Launch &L, const int32_t *ws
     return (L.tail_slots >> SL) & 1u ? ws[SL * kItems * kThreads + r] : 0;
 }
 
-template <int TERM, class B, int NREGS, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int SPLIT, int CARRY, int... KS>
 __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS> &S, const int4 *s_buf, int st,
                                           uint64_t tile,
                                           uint8_t *s_list, uint32_t *s_key, uint32_t *s_sum,
@@ -1675,7 +1675,7 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS> &S, cons
     } else {
         S.live = S.valid;
     }
-    run_steps<B, 0, KS...>(L, S, std::make_integer_sequence<int, kDenseOps>{});
+    run_steps<Dyn, 0, KS...>(L, S, std::make_integer_sequence<int, kDenseOps>{});
 
     if constexpr (kCompact) {
         // warp prefix sum of the live-row counts
@@ -1719,9 +1719,9 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS> &S, cons
             for (; b + 32 <= avail; b += 32) {
                 VRow<NREGS> R = entry(b + lane);
                 if constexpr (use_level2<SPLIT, KS...>(CARRY))
-                    level2_group<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, R, Q, s_bits, s_key, s_sum, direct, acc);
+                    level2_group<TERM, NREGS, SPLIT, CARRY, KS...>(L, R, Q, s_bits, s_key, s_sum, direct, acc);
                 else
-                    sparse_row<TERM, B, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
+                    sparse_row<TERM, Dyn, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
             }
             const uint32_t rem = avail - b;
             if (lane < rem && b + lane >= carry) {  // carry a survivor of this tile
@@ -1741,7 +1741,7 @@ __device__ __forceinline__ void tile_body(const Launch &L, State<NREGS> &S, cons
                 R.live = idx < total;
                 R.r = R.live ? list[idx] : 0;
                 R.grow = tile + (uint64_t)warp * 32 * kItems + R.r;
-                sparse_row<TERM, B, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
+                sparse_row<TERM, Dyn, NREGS, SPLIT, KS...>(L, R, s_bits, s_key, s_sum, direct, acc);
             }
             __syncwarp();
         }
@@ -1807,7 +1807,7 @@ __device__ __forceinline__ void block_flush(const LaunchT &L, uint32_t *s_key, u
     }
 }
 
-template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
 __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES>()) k_dense(const __grid_constant__ Launch L)
 {
     constexpr int kStages = STAGES;
@@ -1850,13 +1850,13 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES>()) k_dense(
         issue_tile<kStages, SS, kItems>(L.slot, L.nstaged, L.n, s_buf, (st + kStages - 1) % kStages,
                                 tile + (kStages - 1) * stride);
         cp_async_wait<kStages - 1>();
-        tile_body<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, S, s_buf, st, tile, s_list, s_key, s_sum, s_bits, direct, acc,
+        tile_body<TERM, NREGS, SPLIT, CARRY, KS...>(L, S, s_buf, st, tile, s_list, s_key, s_sum, s_bits, direct, acc,
                                                    carry, ce, Q);
         st = (st + 1) % kStages;
     }
     cp_async_wait<0>();
     if constexpr (CARRY > 0)
-        drain_carry<TERM, B, NREGS, SPLIT, CARRY, KS...>(L, carry, ce, Q, s_bits, s_key, s_sum, direct, acc);
+        drain_carry<TERM, NREGS, SPLIT, CARRY, KS...>(L, carry, ce, Q, s_bits, s_key, s_sum, direct, acc);
     block_flush<TERM>(L, s_key, s_sum, s_part, acc);
 }
 
@@ -2125,7 +2125,7 @@ struct Span {
 // new descriptor, resets its group table and re-stages the semi-join bitmap.
 // Within a span the tiles go through the same cp.async ring as the
 // single-chain pass.
-template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
 __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES>())
     k_batch(const Launch *__restrict__ launches, const Span *__restrict__ spans, uint32_t n_spans,
             uint32_t *__restrict__ head)
@@ -2192,14 +2192,14 @@ __global__ void __launch_bounds__(kThreads, dense_min_blocks<STAGES>())
                                         (uint64_t)tn * kTile);
             else cp_async_commit();
             cp_async_wait<kStages - 1>();
-            tile_body<TERM, B, NREGS, SPLIT, CARRY, KS...>(s_L, S, s_buf, st, (uint64_t)t * kTile, s_list, s_key, s_sum,
+            tile_body<TERM, NREGS, SPLIT, CARRY, KS...>(s_L, S, s_buf, st, (uint64_t)t * kTile, s_list, s_key, s_sum,
                                                        s_bits, direct, acc, carry, ce, Q);
             st = (st + 1) % kStages;
         }
         cp_async_wait<0>();
         // parked rows belong to this span's chain: run them before the next pull
         if constexpr (CARRY > 0)
-            drain_carry<TERM, B, NREGS, SPLIT, CARRY, KS...>(s_L, carry, ce, Q, s_bits, s_key, s_sum, direct, acc);
+            drain_carry<TERM, NREGS, SPLIT, CARRY, KS...>(s_L, carry, ce, Q, s_bits, s_key, s_sum, direct, acc);
     }
     if (cur != ~0u) block_flush<TERM>(s_L, s_key, s_sum, s_part, acc);
 }
@@ -2264,10 +2264,10 @@ __global__ void __launch_bounds__(kThreads, kLateBlocks)
 // counters, read by sdb_fused_launch_counts).
 std::atomic<uint64_t> g_dense_launches{0}, g_bound_launches{0};
 
-template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
 int launch_stages(const Launch &L, cudaStream_t s)
 {
-    auto kern = k_dense<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
+    auto kern = k_dense<TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
     const int ring = STAGES * kSlots * kThreads * (kItems / 4) * (int)sizeof(int4);
     const int smem = ring + (L.bitmap_ht ? (int)(((L.bitmap_len + 31) / 32) * 4) : 0);
     static sdb::SmemLimit smem_limit;  // one per instantiation
@@ -2282,20 +2282,19 @@ int launch_stages(const Launch &L, cudaStream_t s)
     if (blocks == 0) blocks = 1;
     kern<<<(unsigned)blocks, kThreads, smem, s>>>(L);
     g_dense_launches.fetch_add(1, std::memory_order_relaxed);
-    if (B::bound) g_bound_launches.fetch_add(1, std::memory_order_relaxed);
     return sdb_check_launch("sdb_fused_chain (dense)");
 }
 
 // Ring stages 3 or 2; rows carried between tiles (carry 1; 2: and the second
 // compaction level) only with compaction and a 2-stage ring.
-template <class B, int TERM, int NREGS, int SPLIT, int... KS>
+template <int TERM, int NREGS, int SPLIT, int... KS>
 int launch(const Launch &L, int stages, int carry, cudaStream_t s)
 {
     constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
-    if (stages >= 3) return launch_stages<Dyn, TERM, NREGS, 3, SPLIT, 0, KS...>(L, s);
-    if (kCompact && carry >= 2) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(L, s);
-    if (kCompact && carry == 1) return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(L, s);
-    return launch_stages<Dyn, TERM, NREGS, 2, SPLIT, 0, KS...>(L, s);
+    if (stages >= 3) return launch_stages<TERM, NREGS, 3, SPLIT, 0, KS...>(L, s);
+    if (kCompact && carry >= 2) return launch_stages<TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(L, s);
+    if (kCompact && carry == 1) return launch_stages<TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(L, s);
+    return launch_stages<TERM, NREGS, 2, SPLIT, 0, KS...>(L, s);
 }
 
 // Slot bit of an operand (bit s: column slot s), and the slots an op reads.
@@ -2749,7 +2748,7 @@ struct SingleLauncher {
     template <class B, int TERM, int NREGS, int SPLIT, int... KS>
     int run()
     {
-        return launch<B, TERM, NREGS, SPLIT, KS...>(D, stages, carry, s);
+        return launch<TERM, NREGS, SPLIT, KS...>(D, stages, carry, s);
     }
 };
 
@@ -2771,11 +2770,11 @@ int dispatch(const ChainLaunch &C, int nregs, int term, int compact, int stages,
 }
 
 // One launch of k_batch over the chains of one shape group.
-template <class B, int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
+template <int TERM, int NREGS, int STAGES, int SPLIT, int CARRY, int... KS>
 int batch_stages(const Launch *launches, const Span *spans, uint32_t n_spans, uint32_t *head, uint32_t bitmap_words,
                  cudaStream_t s)
 {
-    auto kern = k_batch<B, TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
+    auto kern = k_batch<TERM, NREGS, STAGES, SPLIT, CARRY, KS...>;
     const int ring = STAGES * kSlots * kThreads * (kItems / 4) * (int)sizeof(int4);
     const int smem = ring + (int)(bitmap_words * 4);
     static sdb::SmemLimit smem_limit;  // one per instantiation
@@ -2788,7 +2787,6 @@ int batch_stages(const Launch *launches, const Span *spans, uint32_t n_spans, ui
     if (blocks == 0) return SDB_OK;
     kern<<<(unsigned)blocks, kThreads, smem, s>>>(launches, spans, n_spans, head);
     g_dense_launches.fetch_add(1, std::memory_order_relaxed);
-    if (B::bound) g_bound_launches.fetch_add(1, std::memory_order_relaxed);
     return sdb_check_launch("sdb_chain_batch_launch");
 }
 
@@ -2806,14 +2804,14 @@ struct BatchLauncher {
     {
         constexpr bool kCompact = SPLIT <= (int)sizeof...(KS);
         if (stages >= 3)
-            return batch_stages<Dyn, TERM, NREGS, 3, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words, s);
+            return batch_stages<TERM, NREGS, 3, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words, s);
         if (kCompact && carry >= 2)
-            return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(launches, spans, n_spans, head,
+            return batch_stages<TERM, NREGS, 2, SPLIT, kCompact ? 2 : 0, KS...>(launches, spans, n_spans, head,
                                                                                    bitmap_words, s);
         if (kCompact && carry == 1)
-            return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(launches, spans, n_spans, head,
+            return batch_stages<TERM, NREGS, 2, SPLIT, kCompact ? 1 : 0, KS...>(launches, spans, n_spans, head,
                                                                                    bitmap_words, s);
-        return batch_stages<Dyn, TERM, NREGS, 2, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words, s);
+        return batch_stages<TERM, NREGS, 2, SPLIT, 0, KS...>(launches, spans, n_spans, head, bitmap_words, s);
     }
 };
 
