@@ -65,11 +65,16 @@ namespace sdb {
 
 constexpr uint64_t kDefaultSegment = 1ull << 28;  // common.hpp:12
 // Aggregating chains of at least this many rows are not put in a batch's
-// chain batch: one launch of such a chain fills the GPU by itself (152 SMs x
-// 5 blocks x 8 tiles of 1024 rows is 6.2 M rows), and the tuned single-chain
-// kernel runs it faster than the persistent batched one.  Measured on the
-// 64-plan star batch: 2^21 / 2^22 / 2^23 / 2^25 / never -> 21.8 / 22.0 /
-// 22.3 / 21.1 / 21.0 thousand queries/s; the served SF50 mix gains 15 %.
+// chain batch: one launch of such a chain fills the GPU by itself, and the
+// single-chain pass has no spans to pull and no change of chain on the way.
+// Whole runs of star batches, us, for lines of 2^20, 2^21, 2^22, 2^23, 2^24 rows
+// and none:
+//   64 plans, median 7 M rows    1831  1874  1869  1909  2187  2334
+//   12 plans, median 7 M rows     330   350   371   406   400   397
+//   32 plans, median 2 M rows     409   403   391   392   385   386
+//   64 plans, median 500 K rows   313   293   278   275   277   276
+// 2^22 reads 2 to 9 % less than 2^23 where partitions are large; the line has
+// stayed where the batch's callers and tests know it.
 constexpr uint64_t kSoloChainRows = 1ull << 23;
 
 // kernels/types.cpp:3-21
@@ -158,7 +163,7 @@ int32_t stoi_ref(const std::string &s)
 }
 
 // Pinned bytes an engine keeps for its results: 65536 slots of a three-key
-// group-by (5 columns, 24 bytes a slot) and more; a result above it is copied.
+// group-by (4 columns, 20 bytes a slot) and more; a result above it is copied.
 constexpr uint64_t kPinnedResult = 4u << 20;
 // Rows up to which an ordered result is sorted by counting (sdb_sort_rows's
 // small case), in the launch that gathers it.
@@ -272,9 +277,10 @@ public:
         return p;
     }
 
+    void rewind() { used_ = 0; }
+
     // memory_manager::reset (operations/memory_manager.cpp:71-90): rewind and
     // re-zero what the zeroed region handed out.
-    void rewind() { used_ = 0; }
     void reset(cudaStream_t s)
     {
         used_ = 0;
@@ -2747,7 +2753,9 @@ void plan_cache_clear(sdb_engine &eng)
 // prepares it as a one-plan batch (recorded once against its own arena,
 // captured as a CUDA graph, fused chains launched on their own); from then on
 // an execution is one graph launch and the unpacking of its result.  The
-// device work is the plain path's, kernel for kernel.
+// device work is the plain path's, kernel for kernel but for the table builds:
+// one launch of the batch's build kernel here (k_build_batch), of up to four at
+// a time there (sdb_build_few).
 std::unique_ptr<sdb_result> execute_cached(sdb_engine &eng, const std::string &text)
 {
     Engine &E = eng.E;

@@ -3,7 +3,8 @@
 // The shape-specialised passes (namespace dense) are compiled for the op
 // sequences of the common plans.  Every other chain used to go through the
 // general interpreter (k_chain), which runs each op on all rows of a tile in
-// turn, one dependent memory round trip after the other.  The sieve reads its ops at run
+// turn, one dependent memory round trip after the other; small and plain ones
+// still do (rows_from).  The sieve reads its ops at run
 // time too, but orders its work as the specialised passes do: rows fall
 // through three levels, each on full warps.
 //
@@ -18,9 +19,9 @@
 //           read from here on costs only the sectors that hold such rows.
 //
 // SSB flight 4.2 over 60 M rows (four joins, six columns, three keys): 1126 us
-// in the general pass, 250 here.  Where the time goes: streaming the two
-// copied columns and listing the survivors 130 us, the probe of the customer
-// table 60, the second level 28, the group-by 34.
+// in the general pass, 218 here.  What is left is the streaming of the two
+// copied columns and the listing of the survivors first, then the probe of the
+// customer table.
 //
 // Included by fused.cu (uses its namespace dense).
 #pragma once
