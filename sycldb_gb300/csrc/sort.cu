@@ -669,8 +669,9 @@ __device__ __forceinline__ bool pass_tile(const PassArgs &a, const PassPlan &pla
 //
 // 16.8 M pairs: 100 to 103 us a pass (2.6 TB/s of the 16 bytes a pair moves), from
 // 210 us for the count, the three scans and the scatter that it replaces.
-// Bound by shared memory (half its cycles) and issue: the ballots are a third
-// of 115 warp instructions per 32 pairs.  __match_any_sync in their place
+// Bound by latency at two blocks an SM: barriers first among the waits, issue in
+// 42 % of the cycles (the ballots are a third of 98 warp instructions per 32
+// pairs), shared memory in 38 %.  __match_any_sync in their place
 // took 57 cycles a step on its one unit per SM (155 us).  Tiles of 4096, 5120,
 // 8192 pairs, 256, 512 and 1024 threads: 2 to 10 % slower.
 template <int SHIFT>
