@@ -133,3 +133,14 @@ def test_dense_op_reads_an_unwritten_register(shape, reg_at, n):
     want = same(make(np.random.default_rng(n + reg_at), shape, n, reg_at))
     assert not any(w.any() for w in want[:2])  # no row passes
     release()
+
+
+@pytest.mark.parametrize("shape", sorted(SHAPES))
+@pytest.mark.parametrize("n", [1, 2047, 60_013])
+def test_every_shape_gives_the_sums_and_the_keys(shape, n):
+    """Each shape at the edges of its tiles, a few, most and all of the rows
+    left: sums, occupied slots and the keys their first writers store."""
+    for hits in (0.05, 0.7, 1.0):
+        d = make(np.random.default_rng(n), shape, n, hits=hits)
+        same(d)
+        release()
